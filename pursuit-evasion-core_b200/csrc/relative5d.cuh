@@ -82,8 +82,11 @@ struct Rel5Tile {
 // Shared memory the fast kernel needs for a tile.
 size_t rel5_fast_smem_bytes(const Rel5Grid &g, const Rel5Tile &t);
 
-// Default tile for a grid (rows chosen so rows * xp/4 threads ~ 256).
+// Default tile for a grid: the one of least estimated stage time.
 Rel5Tile rel5_default_tile(const Rel5Grid &g);
+
+// Estimated time of one float32 stage in tiles `t`, microseconds.
+double rel5_tile_cost(const Rel5Grid &g, const Rel5Tile &t);
 
 // Resident CTAs per SM of the most recent fast-stage launch.
 int rel5_last_resident_ctas();

@@ -41,89 +41,15 @@
 #include <algorithm>
 #include <cstdio>
 
-#include "bulk_copy.cuh"
 #include "relative5d.cuh"
 #include "relative5d_eno_f32.cuh"
+#include "relative5d_ring.cuh"
 
 namespace pe {
 namespace {
 
 using namespace eno32;
-using namespace bulk;
-
-constexpr int OWN_SLOTS = 8;   // own-plane ring (power of two)
-constexpr int STEP_SLOTS = 2;  // neighbour sets and step barriers
-constexpr int NEIGHBOURS = 8;  // vE-2, vE-1, vE+1, vE+2, vP-2, vP-1, vP+1, vP+2
-// a neighbour set also holds, on RK2 stage 2, the item's rows of the
-// stage's old value V (the blend partner), prefetched with the neighbours
-constexpr int NB_PLANES = NEIGHBOURS + 1;
-constexpr int MAX_THREADS = 512;
-constexpr int TARGET_THREADS = 256;  // launch bound: two CTAs of 256 per SM
-constexpr int MIN_ITEM_STEPS = 4;    // own-ring reuse needs items of >= 4 headings
-// A try waits for up to the hardware's own time limit before it returns
-// false; a wait gives up after WAIT_LIMIT tries.  (On the 89M-cell grid a
-// suspend-time hint of 1 us per try measured 0.8 % slower, and a
-// %globaltimer bound in the loop 1.3 % slower.)
-constexpr unsigned WAIT_LIMIT = 1u << 21;
-
-// Bounded wait for one mbarrier phase.  Returns false (and flags the handle)
-// when the limit is reached.
-__device__ __forceinline__ bool wait_phase(uint64_t *bar, uint32_t parity,
-                                           unsigned int *timeout_flag) {
-  return bulk::wait_phase(bar, parity, timeout_flag, WAIT_LIMIT);
-}
-
-struct FastArgs {
-  Rel5Grid g;
-  Rel5Stage s;
-  int rows, psi_chunk, slabs, chunks, xc, consumer_warps, items;
-  int vp_first, vp_count;  // the vP slabs this launch updates (a shard's own)
-  float ihx, ihp, ihv, ihe;
-  float dt;
-};
-
-// Shared memory layout of one CTA.
-struct SmemLayout {
-  int own_floats, nb_floats;
-  int own_off, nb_off;                 // floats
-  int bar_off, red_off, trig_off;      // bytes
-  int bytes;
-};
-
-__host__ __device__ inline SmemLayout smem_layout(int rows, int xp, int headings) {
-  SmemLayout L;
-  L.own_floats = (rows + 4) * xp;
-  L.nb_floats = rows * xp;
-  L.own_off = 0;
-  L.nb_off = OWN_SLOTS * L.own_floats;
-  L.bar_off = 4 * (L.nb_off + STEP_SLOTS * NB_PLANES * L.nb_floats);
-  L.red_off = L.bar_off + 8 * 2 * STEP_SLOTS;
-  L.trig_off = L.red_off + 4 * (MAX_THREADS / 32);
-  L.bytes = L.trig_off + 4 * 2 * headings;
-  return L;
-}
-
-// One work item: `rows` y rows (from y0) of one (vP, vE) pair over `steps`
-// headings from p0.  Items are numbered heading chunk first, so that the
-// CTAs resident at any moment share the planes of a few headings in L2.
-struct Item {
-  int iv, ie, y0, r_eff, p0, steps;
-};
-
-__device__ __forceinline__ Item decode_item(const FastArgs &a, int idx) {
-  Item it;
-  const int slab = idx % a.slabs;
-  idx /= a.slabs;
-  it.ie = idx % a.g.nve;
-  idx /= a.g.nve;
-  it.iv = a.vp_first + idx % a.vp_count;
-  const int chunk = idx / a.vp_count;
-  it.y0 = slab * a.rows;
-  it.r_eff = min(a.rows, a.g.nx - it.y0);
-  it.p0 = chunk * a.psi_chunk;
-  it.steps = min(a.psi_chunk, a.g.nh - it.p0);
-  return it;
-}
+using namespace ring;
 
 __device__ __forceinline__ float2 ld2(const float *p) {
   return *reinterpret_cast<const float2 *>(p);
@@ -166,14 +92,14 @@ __device__ __forceinline__ void sum_jump4(float4 m2, float4 m1, float4 v, float4
 // XR = nx mod 4 places the x end rules (see slopes_x_fixed).
 template <int ORDER, int BLEND, int XR, int XPC, int RC>
 __global__ void __launch_bounds__(TARGET_THREADS, 2)
-    rel5_stage_kernel(const FastArgs a) {
+    rel5_stage_kernel(const RingArgs a) {
   extern __shared__ __align__(128) float smem[];
   const Rel5Grid &g = a.g;
   // XPC / RC: the row pitch and tile rows at compile time (0: from the
   // arguments), so that every shared-memory offset is an immediate
   const int R = RC ? RC : a.rows, XP = XPC ? XPC : g.xp;
   const int XC = XPC ? XPC / 4 : a.xc;
-  const SmemLayout L = smem_layout(R, XP, g.nh);
+  const SmemLayout L = smem_layout(R, XP, 8 * g.nh);
   float *own = smem + L.own_off;  // [8][R+4][XP]
   float *nbr = smem + L.nb_off;   // [2][9][R][XP]
   char *raw = reinterpret_cast<char *>(smem);
@@ -208,67 +134,7 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
   bool alive = true;
 
   if (producer) {
-    if (lane == 0) {
-      unsigned og = 0, gs = 0;  // own planes / steps issued so far
-      for (int idx = blockIdx.x; idx < a.items && alive; idx += gridDim.x) {
-        const Item it = decode_item(a, idx);
-        const int row_lo = max(0, it.y0 - 2), row_hi = min(g.nx, it.y0 + it.r_eff + 2);
-        const uint32_t own_bytes = (uint32_t)((row_hi - row_lo) * XP * 4);
-        const float *own_src = a.s.src + (int64_t)row_lo * XP;
-        const int own_dst = (row_lo - (it.y0 - 2)) * XP;
-        const uint32_t nb_bytes = (uint32_t)(it.r_eff * XP * 4);
-        int nb_e[NEIGHBOURS], nb_v[NEIGHBOURS], nb_count = 0;
-        {
-          const int de[NEIGHBOURS] = {-2, -1, 1, 2, 0, 0, 0, 0};
-          const int dv[NEIGHBOURS] = {0, 0, 0, 0, -2, -1, 1, 2};
-          for (int q = 0; q < NEIGHBOURS; q++) {
-            nb_e[q] = it.ie + de[q];
-            nb_v[q] = it.iv + dv[q];
-            const bool ok = nb_e[q] >= 0 && nb_e[q] < g.nve && nb_v[q] >= 0 && nb_v[q] < g.nvp;
-            if (!ok) nb_e[q] = -1;
-            nb_count += ok;
-          }
-        }
-        for (int k = 0; k < it.steps; k++) {
-          const int slot = (int)(gs & 1u);
-          // the slot's previous step (gs - 2) must be released first
-          if (gs >= STEP_SLOTS)
-            alive = wait_phase(&empty[slot], ((gs >> 1) - 1) & 1u, timeout);
-          if (!alive) break;
-          fence_async_shared();
-          const int d_first = k == 0 ? -2 : k + 2;
-          const int n_own = k + 3 - d_first;
-          mbar_expect_tx(&full[slot], (uint32_t)n_own * own_bytes +
-                                          nb_bytes * (nb_count + (BLEND ? 1 : 0)));
-          for (int d = d_first; d <= k + 2; d++) {
-            const int psi = ((it.p0 + d) % g.nh + g.nh) % g.nh;
-            bulk_load(own + (og & (OWN_SLOTS - 1)) * L.own_floats + own_dst,
-                      own_src + plane_index(it.iv, it.ie, psi) * PP, own_bytes, &full[slot]);
-            og++;
-          }
-          float *set = nbr + slot * NB_PLANES * L.nb_floats;
-          for (int q = 0; q < NEIGHBOURS; q++)
-            if (nb_e[q] >= 0)
-              bulk_load(set + q * L.nb_floats,
-                        a.s.src + plane_index(nb_v[q], nb_e[q], it.p0 + k) * PP +
-                            (int64_t)it.y0 * XP,
-                        nb_bytes, &full[slot]);
-          // the blend partner V of this step's rows: read here before any
-          // consumer writes them (they wait for this set first)
-          if (BLEND)
-            bulk_load(set + NEIGHBOURS * L.nb_floats,
-                      a.s.dst + plane_index(it.iv, it.ie, it.p0 + k) * PP +
-                          (int64_t)it.y0 * XP,
-                      nb_bytes, &full[slot]);
-          gs++;
-        }
-      }
-      // After a timeout, let the copies already issued (the last two steps'
-      // sets at most) land before the CTA exits.
-      if (!alive)
-        for (unsigned q = gs > STEP_SLOTS ? gs - STEP_SLOTS : 0; q < gs; q++)
-          wait_phase(&full[q & 1u], (q >> 1) & 1u, timeout);
-    }
+    if (lane == 0) produce<BLEND>(a, L, own, nbr, full, empty, XP);
   } else {
     const int r = tid / XC, c = tid % XC;
     const int x0 = 4 * c;
@@ -577,7 +443,7 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
 int g_last_resident = 0;
 
 template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0>
-cudaError_t launch_xr(const FastArgs &args, size_t smem, int threads, cudaStream_t stream) {
+cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
   // Resident CTAs per SM for this (shared memory, block size); recomputed
   // when either changes.
   static int configured_smem = 0, configured_threads = 0;
@@ -604,7 +470,7 @@ cudaError_t launch_xr(const FastArgs &args, size_t smem, int threads, cudaStream
 }
 
 template <int ORDER, int BLEND>
-cudaError_t launch(const FastArgs &args, size_t smem, int threads, cudaStream_t stream) {
+cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
   // the 65-position grids (68-float rows) at the default 13-row tile, with
   // compile-time offsets (5 % faster on the 89M-cell grid, B200)
   if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13)
@@ -680,27 +546,54 @@ cudaError_t rel5_unpack(const Rel5Grid &g, const float *dense, float *padded,
 int rel5_last_resident_ctas() { return g_last_resident; }
 
 size_t rel5_fast_smem_bytes(const Rel5Grid &g, const Rel5Tile &t) {
-  return (size_t)smem_layout(t.rows, g.xp, g.nh).bytes;
+  return (size_t)smem_layout(t.rows, g.xp, 8 * g.nh).bytes;
 }
 
+// Time of one stage in tiles `t`, in microseconds of the float32 kernel on a
+// B200: the items' heading steps (each item also pays about 3 steps to start
+// its rings) over the CTAs that fit the SMs by shared memory and registers.
+// A step of the CTAs of one SM costs 0.1 us per consumer warp (throughput),
+// and not less than 0.9 us (the latency of one step); the y halo rows add a
+// little (17-row items beat 7-row ones by 6 % at 49x36x15x15).  Measured stages lie
+// within 20 % of it from 16,200 to 89 M cells.
+double rel5_tile_cost(const Rel5Grid &g, const Rel5Tile &t) {
+  const int kSms = 148, kRegs = 128;
+  const int warps = (t.rows * (g.xp / 4) + 31) / 32;
+  const int smem = (int)rel5_fast_smem_bytes(g, t) + 1024;
+  const int resident = std::max(
+      1, std::min({227 * 1024 / smem, 65536 / (kRegs * 32 * (warps + 1)), 32}));
+  const int64_t slabs = (g.nx + t.rows - 1) / t.rows;
+  const int64_t chunks = (g.nh + t.psi_chunk - 1) / t.psi_chunk;
+  const int64_t items = slabs * g.nve * (g.own_n > 0 ? g.own_n : g.nvp) * chunks;
+  auto step = [&](int64_t ctas) { return std::max(0.9, 0.1 * warps * (double)ctas); };
+  const int64_t full = items / (kSms * resident), rest = items % (kSms * resident);
+  return (t.psi_chunk + 3) * (1 + 0.3 / t.rows) *
+         (full * step(resident) + (rest ? step((rest + kSms - 1) / kSms) : 0.0));
+}
+
+// The tile of least rel5_tile_cost, the larger one where two cost the same
+// (fewer halo rows).  Heading chunks stay at 24 or below: the CTAs resident
+// at a time then share the planes of a few headings in L2 (at 65x48x21x21
+// chunks of 48 measured 3 % slower than 24).  The rule before this took the
+// rows with the fewest idle rows at 24 headings: it gave one-row items on 41
+// positions (534 us per RK2 step, 156 us now) and left most SMs idle on small
+// grids (17x12x7x7: one item per speed pair, 17 us per stage, 8 us now).
 Rel5Tile rel5_default_tile(const Rel5Grid &g) {
-  const int xc = g.xp / 4;
-  Rel5Tile t{1, 8};
-  // rows: at most 7 consumer warps, fewest idle rows, then most rows.
-  int best_waste = 1 << 30;
-  for (int rows = 1; rows * xc <= TARGET_THREADS - 32 && rows <= g.nx; rows++) {
-    const int slabs = (g.nx + rows - 1) / rows;
-    const int waste = slabs * rows - g.nx;
-    if (waste < best_waste || (waste == best_waste && rows > t.rows)) {
-      best_waste = waste;
-      t.rows = rows;
+  Rel5Tile best{1, std::min(g.nh, 24)};
+  double best_cost = 1e300;
+  for (int rows = 1; rows <= g.nx; rows++)
+    for (int chunks = 1; chunks <= g.nh / MIN_ITEM_STEPS; chunks++) {
+      const Rel5Tile t{rows, (g.nh + chunks - 1) / chunks};
+      if (t.psi_chunk > 24 || !rel5_tile_valid(g, t)) continue;
+      const double cost = rel5_tile_cost(g, t);
+      if (cost < best_cost * (1 - 1e-9) ||
+          (cost < best_cost * (1 + 1e-9) &&
+           t.rows * t.psi_chunk >= best.rows * best.psi_chunk)) {
+        best = t;
+        best_cost = std::min(cost, best_cost);
+      }
     }
-  }
-  // Heading chunks of about 24 (fastest on the 65x48x21x21 grid, B200),
-  // balanced so that the last chunk is not short.
-  const int chunks = (g.nh + 23) / 24;
-  t.psi_chunk = (g.nh + chunks - 1) / chunks;
-  return t;
+  return best;
 }
 
 bool rel5_tile_valid(const Rel5Grid &g, const Rel5Tile &t) {
@@ -717,23 +610,7 @@ bool rel5_tile_valid(const Rel5Grid &g, const Rel5Tile &t) {
 cudaError_t rel5_stage_f32(const Rel5Grid &g, const Rel5Tile &t,
                            const Rel5Stage &s, int blend, cudaStream_t stream) {
   if (!rel5_tile_valid(g, t)) return cudaErrorInvalidConfiguration;
-  FastArgs args;
-  args.g = g;
-  args.s = s;
-  args.rows = t.rows;
-  args.psi_chunk = t.psi_chunk;
-  args.xc = g.xp / 4;
-  args.consumer_warps = (t.rows * args.xc + 31) / 32;
-  args.slabs = (g.nx + t.rows - 1) / t.rows;
-  args.chunks = (g.nh + t.psi_chunk - 1) / t.psi_chunk;
-  args.vp_first = g.own_n > 0 ? g.own_lo : 0;
-  args.vp_count = g.own_n > 0 ? g.own_n : g.nvp;
-  args.items = args.slabs * g.nve * args.vp_count * args.chunks;
-  args.ihx = (float)(1.0 / g.dx);
-  args.ihp = (float)(1.0 / g.dphi);
-  args.ihv = (float)(1.0 / g.dvp);
-  args.ihe = (float)(1.0 / g.dve);
-  args.dt = (float)s.dt;
+  const RingArgs args = ring_args(g, t, s);
   const int threads = 32 * (args.consumer_warps + 1);
   const size_t smem = rel5_fast_smem_bytes(g, t);
   if (g.order == 1) return launch<1, 0>(args, smem, threads, stream);
