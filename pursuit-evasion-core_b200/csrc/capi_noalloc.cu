@@ -146,7 +146,7 @@ extern "C" int pe_relative_step_noalloc(const pe_relative_params *params,
   if (g.order == 1) {
     s.src = field_in;
     s.dst = field_out;
-    PE_CUDA_TRY(pe::rel5_stage_f64(g, s, 0, stream));
+    PE_CUDA_TRY(pe::rel5_stage_f64(g, pe::Rel5Tile{0, 0}, s, 0, stream));
     pe::count_launches(1);
   } else {
     // Stage 2 averages with the old value read from its output buffer.
@@ -154,10 +154,10 @@ extern "C" int pe_relative_step_noalloc(const pe_relative_params *params,
                                 cudaMemcpyDeviceToDevice, stream));
     s.src = field_in;
     s.dst = stage;
-    PE_CUDA_TRY(pe::rel5_stage_f64(g, s, 0, stream));
+    PE_CUDA_TRY(pe::rel5_stage_f64(g, pe::Rel5Tile{0, 0}, s, 0, stream));
     s.src = stage;
     s.dst = field_out;
-    PE_CUDA_TRY(pe::rel5_stage_f64(g, s, 1, stream));
+    PE_CUDA_TRY(pe::rel5_stage_f64(g, pe::Rel5Tile{0, 0}, s, 1, stream));
     pe::count_launches(2);
   }
   pe::Rel5Stats host{};

@@ -85,7 +85,7 @@ int launch_stage(pe_relative *h, int stage, const float *src, float *dst,
   cudaEvent_t e0 = h->timer.begin(h->stream);
   const cudaError_t err =
       h->p.precision == PE_LOCAL_F64
-          ? pe::rel5_stage_f64(h->g, s, blend, h->stream)
+          ? pe::rel5_stage_f64(h->g, h->tile, s, blend, h->stream)
           : pe::rel5_stage_f32(h->g, h->tile, s, blend, h->stream);
   if (err != cudaSuccess) return pe::cuda_fail(err, "relative stage launch");
   pe::count_launches(1);

@@ -241,7 +241,7 @@ int pe_relative_shard_stage(pe_relative_shard *h, int32_t stage, double dt) {
   s.t = h->t;
   s.stats = h->stats;
   PE_CUDA_TRY(h->p.precision == PE_LOCAL_F64
-                  ? pe::rel5_stage_f64(h->g, s, blend, h->stream)
+                  ? pe::rel5_stage_f64(h->g, h->tile, s, blend, h->stream)
                   : pe::rel5_stage_f32(h->g, h->tile, s, blend, h->stream));
   pe::count_launches(1);
   h->last = s.dst;

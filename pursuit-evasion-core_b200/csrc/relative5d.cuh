@@ -101,8 +101,14 @@ cudaError_t rel5_stage_f32(const Rel5Grid &g, const Rel5Tile &t,
 
 // Exact path: double local arithmetic in the reference's operation order,
 // built without contraction so it reproduces native_relative.cpp bit for bit.
-cudaError_t rel5_stage_f64(const Rel5Grid &g, const Rel5Stage &s, int blend,
+cudaError_t rel5_stage_f64(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s, int blend,
                            cudaStream_t stream);
+
+// The tiled form of the exact path (relative5d_tiled_exact.cu) and whether it
+// takes this layout, tile and these buffers.
+bool rel5_walk_exact_applies(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s);
+cudaError_t rel5_stage_f64_tiled(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s,
+                                 int blend, cudaStream_t stream);
 
 // Double storage: the exact stage with double values in a dense layout
 // (g.xp == g.nx), no arrival times -- the FP64 oracle (po_rel_stage_f64 of

@@ -73,8 +73,9 @@ cudaError_t rel5_stage_f64_storage(const Rel5Grid &g, const Rel5Stage &s, int bl
   return cudaGetLastError();
 }
 
-cudaError_t rel5_stage_f64(const Rel5Grid &g, const Rel5Stage &s, int blend,
+cudaError_t rel5_stage_f64(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s, int blend,
                            cudaStream_t stream) {
+  if (rel5_walk_exact_applies(g, t, s)) return rel5_stage_f64_tiled(g, t, s, blend, stream);
   const int threads = 128;
   const int slabs = g.own_n > 0 ? g.own_n : g.nvp;
   const dim3 grid((g.nx * g.nx + threads - 1) / threads, slabs * g.nve, g.nh);

@@ -1,0 +1,230 @@
+// Relative 5D ENO/LF stage, exact variant, tiled: the results of
+// relative5d_exact.cu bit for bit (double local arithmetic in the order of
+// native_relative.cpp:38-67, :124-172, float32 storage), on the streaming
+// scheme of the float32 stage (relative5d_ring.cuh): a work item is `rows` y
+// rows of one (vP, vE) pair over a chunk of headings, a consumer thread owns
+// 4 consecutive x cells of a row and walks the headings, a producer warp
+// streams the planes by bulk copies.  Compiled with -fmad=false.
+//
+// The thread-per-cell kernel forms 25 quotients, 10 selections and 21
+// conversions per cell, with a range check on every quotient; here the
+// heading axis' are carried from step to step, the x axis' shared inside the
+// chunk, and the range checks are replaced by one test of the result
+// (relative5d_exact_walk.cuh): about 165 double operations per cell, which
+// bound it (64 per clock and SM): 1.77 ms per stage at 65x48x21x21 (4.0 ms
+// for the thread-per-cell kernel), of which the double operations are 0.85.
+#include "relative5d_exact_walk.cuh"
+#include "relative5d_ring.cuh"
+
+namespace pe {
+namespace {
+
+using namespace ring;
+
+// heading (cos, sin) pairs and x positions, in double
+__host__ __device__ inline int table_bytes(const Rel5Grid &g) { return 16 * g.nh + 8 * g.xp; }
+
+template <int ORDER, int BLEND, int XR, int XPC, int RC>
+__global__ void __launch_bounds__(TARGET_THREADS, 2)
+    rel5_walk_exact_kernel(const __grid_constant__ RingArgs a) {
+  extern __shared__ __align__(128) float smem[];
+  const Rel5Grid &g = a.g;
+  const int R = RC ? RC : a.rows, XP = XPC ? XPC : g.xp;
+  const int XC = XPC ? XPC / 4 : a.xc;
+  const SmemLayout L = smem_layout(R, XP, table_bytes(g));
+  float *own = smem + L.own_off;  // [8][R+4][XP]
+  float *nbr = smem + L.nb_off;   // [2][9][R][XP]
+  char *raw = reinterpret_cast<char *>(smem);
+  uint64_t *full = reinterpret_cast<uint64_t *>(raw + L.bar_off);
+  uint64_t *empty = full + STEP_SLOTS;
+  double2 *trig = reinterpret_cast<double2 *>(raw + L.trig_off);  // [nh] cos, sin
+  double *xtab = reinterpret_cast<double *>(trig + g.nh);         // [xp]
+
+  const int64_t PP = (int64_t)g.nx * XP;  // plane pitch
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool producer = warp == a.consumer_warps;
+  unsigned int *timeout = &a.s.stats->timeout;
+
+  if (tid == 0) {
+    for (int i = 0; i < STEP_SLOTS; i++) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 32 * a.consumer_warps);
+    }
+    fence_barrier_init();
+  }
+  for (int k = tid; k < g.nh; k += blockDim.x)
+    trig[k] = make_double2(__ldg(a.s.cs + k), __ldg(a.s.sn + k));
+  for (int k = tid; k < XP; k += blockDim.x) xtab[k] = -g.extent + k * g.dx;
+  __syncthreads();
+
+  bool bad = false;
+  exact::ChangeMax change;
+
+  if (producer) {
+    if (lane == 0) produce<BLEND>(a, L, own, nbr, full, empty, XP);
+  } else {
+    const int r = tid / XC, c = tid % XC;
+    const int x0 = 4 * c;
+    constexpr int KP = (XR + 2) & 3, IEND = (XR + 3) & 3;
+    const bool first = x0 == 0;
+    const bool kend = x0 == g.nx - 2 - KP;
+    const bool iend = x0 == g.nx - 1 - IEND;
+    const int valid = iend ? IEND + 1 : 4;
+    const exact::AxisSteps st{exact::axis_step(g.dx, g.rdx, g.rdx2),
+                              exact::axis_step(g.dphi, g.rdphi, g.rdphi2),
+                              exact::axis_step(g.dvp, g.rdvp, g.rdvp2),
+                              exact::axis_step(g.dve, g.rdve, g.rdve2)};
+    const int ctr = (r + 2) * XP + x0;  // this chunk in an own slot
+    const int nbo = r * XP + x0;        // this chunk in a neighbour slot
+    bool alive = true;
+    unsigned og = 0, gs = 0;
+
+    for (int idx = blockIdx.x; idx < a.items && alive; idx += gridDim.x) {
+      const Item it = decode_item(a, idx);
+      const bool active = r < it.r_eff;
+      // warps holding a row within two of a y end take the general y rules
+      const int rw0 = (32 * warp) / XC;
+      const int rw1 = min((32 * warp + 31) / XC, it.r_eff - 1);
+      exact::ItemCoef q;
+      q.iy = it.y0 + r;
+      q.nx = g.nx;
+      q.iv = it.iv;
+      q.nvp = g.nvp;
+      q.ie = it.ie;
+      q.nve = g.nve;
+      q.y_general = it.y0 + rw0 < 2 || it.y0 + rw1 + 2 >= g.nx;
+      q.v_general = it.iv < 2 || it.iv + 2 >= g.nvp;
+      q.e_general = it.ie < 2 || it.ie + 2 >= g.nve;
+      q.y = -g.extent + q.iy * g.dx;
+      q.vp = g.vp_lo + it.iv * g.dvp;
+      q.ve = g.ve_lo + it.ie * g.dve;
+      q.wp = fabs(q.vp) * g.curv_p;
+      q.we = fabs(q.ve) * g.curv_e;
+      q.acc_p = g.acc_p;
+      q.acc_e = g.acc_e;
+      q.dt = a.s.dt;
+      const unsigned base = og;  // issue index of own plane d = -2
+      og += it.steps + 4;
+      int64_t j = (((int64_t)(it.iv - g.slab_lo) * g.nve + it.ie) * g.nh + it.p0) * PP +
+                  (int64_t)q.iy * XP + x0;
+      auto own_at = [&](unsigned p) -> const float * {
+        return own + (p & (OWN_SLOTS - 1)) * L.own_floats + ctr;
+      };
+      auto own4 = [&](unsigned p) { return *reinterpret_cast<const float4 *>(own_at(p)); };
+
+      // Step 0's set holds planes -2..2: start the heading differences.
+      if (alive) alive = wait_phase(&full[gs & 1u], (gs >> 1) & 1u, timeout);
+      exact::HeadingCarry<ORDER> carry;
+      if (active)  // lanes past the item's rows read nothing
+        carry.start(own4(base), own4(base + 1), own4(base + 2), own4(base + 3), st.psi);
+
+#pragma unroll 1
+      for (int k = 0; k < it.steps; k++) {
+        const unsigned slot = gs & 1u;
+        if (k > 0 && alive) alive = wait_phase(&full[slot], (gs >> 1) & 1u, timeout);
+        if (active && alive) {
+          const float *o0 = own_at(base + k + 2);  // centre plane k
+          const float *nb = nbr + slot * NB_PLANES * L.nb_floats + nbo;
+          const float4 C = *reinterpret_cast<const float4 *>(o0);
+          const double2 cssn = trig[it.p0 + k];
+          double H[4];
+          exact::walk_hamiltonian<ORDER, XR>(
+              *reinterpret_cast<const float2 *>(o0 - 2), C,
+              *reinterpret_cast<const float2 *>(o0 + 4), own4(base + k + 3),
+              own4(base + k + 4), o0, XP, nb, L.nb_floats, first, kend, iend, xtab + x0,
+              cssn.x, cssn.y, q, st, carry, H);
+          const float4 P =
+              BLEND ? *reinterpret_cast<const float4 *>(nb + NEIGHBOURS * L.nb_floats) : C;
+          bad |= exact::walk_update<ORDER, BLEND>(g, a.s, x0, it.p0 + k, j, valid, q,
+                                                  xtab + x0, C, P, H, change);
+        }
+        mbar_arrive(&empty[slot]);  // release this step's set
+        gs++;
+        j += PP;
+      }
+    }
+  }
+
+  // Block reductions: non-finite flag, largest change and increase.
+  if (__syncthreads_or(bad) && tid == 0) atomicOr(&a.s.stats->nonfinite, 1u);
+  if (BLEND || ORDER == 1) {
+    double m_abs = change.abs_max, m_up = change.up_max;
+    for (int off = 16; off > 0; off >>= 1) {
+      m_abs = fmax(m_abs, __shfl_xor_sync(0xffffffffu, m_abs, off));
+      m_up = fmax(m_up, __shfl_xor_sync(0xffffffffu, m_up, off));
+    }
+    if (lane == 0) {
+      exact::atomic_max_nonneg(&a.s.stats->residual, m_abs);
+      exact::atomic_max_nonneg(&a.s.stats->increase, m_up);
+    }
+  }
+}
+
+template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0>
+cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
+  auto kernel = rel5_walk_exact_kernel<ORDER, BLEND, XR, XPC, RC>;
+  // co-resident CTAs of the last (device, shared memory, block size) this
+  // thread launched
+  struct Shape {
+    int device = -1, smem = 0, threads = 0, ctas = 0;
+  };
+  static thread_local Shape last;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  if (last.device != device || last.smem != (int)smem || last.threads != threads) {
+    int sms = 0, resident = 0;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    if (resident < 1) return cudaErrorInvalidConfiguration;
+    last = Shape{device, (int)smem, threads, sms * resident};
+  }
+  kernel<<<std::min(args.items, last.ctas), threads, smem, stream>>>(args);
+  return cudaGetLastError();
+}
+
+template <int ORDER, int BLEND>
+cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
+  if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13)
+    return launch_xr<ORDER, BLEND, 1, 68, 13>(args, smem, threads, stream);
+  switch (args.g.nx & 3) {
+    case 0: return launch_xr<ORDER, BLEND, 0>(args, smem, threads, stream);
+    case 1: return launch_xr<ORDER, BLEND, 1>(args, smem, threads, stream);
+    case 2: return launch_xr<ORDER, BLEND, 2>(args, smem, threads, stream);
+    default: return launch_xr<ORDER, BLEND, 3>(args, smem, threads, stream);
+  }
+}
+
+}  // namespace
+
+// The tiled kernel takes the padded layout on 16-byte bounds, in a tile whose
+// rings and tables fit, where it is the faster one: its stage takes about 3.4
+// times the float32 stage's, the thread-per-cell stage 4 us and 45 us per
+// million cells (B200: 17x12x7x7 39 against 29 us per RK2 step, 21x16x9x9 63
+// against 66, 33x24x11x11 199 against 293, 65x48x21x21 3550 against 8000).
+bool rel5_walk_exact_applies(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s) {
+  if (g.xp % 4 != 0 || g.sy != g.xp ||
+      ((reinterpret_cast<uintptr_t>(s.src) | reinterpret_cast<uintptr_t>(s.dst)) & 15) != 0)
+    return false;
+  if (!rel5_tile_valid(g, t) ||
+      smem_layout(t.rows, g.xp, table_bytes(g)).bytes > 227 * 1024)
+    return false;
+  const double cells = (double)g.se * g.nve * (g.own_n > 0 ? g.own_n : g.nvp);
+  return 3.4 * rel5_tile_cost(g, t) < 4.0 + 45e-6 * cells;
+}
+
+cudaError_t rel5_stage_f64_tiled(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s,
+                                 int blend, cudaStream_t stream) {
+  const RingArgs args = ring_args(g, t, s);
+  const int threads = 32 * (args.consumer_warps + 1);
+  const size_t smem = (size_t)smem_layout(t.rows, g.xp, table_bytes(g)).bytes;
+  if (g.order == 1) return launch<1, 0>(args, smem, threads, stream);
+  if (blend) return launch<2, 1>(args, smem, threads, stream);
+  return launch<2, 0>(args, smem, threads, stream);
+}
+
+}  // namespace pe
