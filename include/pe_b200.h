@@ -628,6 +628,49 @@ int pe_mlp_encode_world_nodes(const float *table, const int64_t *idx, int n,
                               double e_max, void *feat, int ld, float *target,
                               void *cuda_stream);
 
+/* The whole network (hidden width 256, input width 128, up to 8 layers) in
+ * few launches (csrc/mlp_fused.cu); the arithmetic and the buffers are those
+ * of the entry points above. */
+typedef struct pe_mlp_net {
+  int32_t layers, hidden, in_width;
+  const void *w16[8];   /* bf16 weights, layer l [hidden][in] */
+  const void *w16t[8];  /* their transposes [in][hidden] (backward only) */
+  const float *b[8];    /* biases [hidden] */
+  const float *w_out, *b_out;
+} pe_mlp_net;
+/* Forward pass over bf16 features [rows][128]: activations h[l] and, where
+ * z[l] is not NULL (z itself may be NULL), pre-activations, y, and with a
+ * target dy and loss as pe_mlp_head_forward.  rows a multiple of 128. */
+int pe_mlp_forward(const pe_mlp_net *net, const void *feat, int rows, float *const *z,
+                   void *const *h, const float *target, float *y, float *dy, float *loss,
+                   void *cuda_stream);
+/* Activation gradients dz[l], and the weight, bias and head gradients added
+ * to gw[l] [hidden][in], gb[l], gw_out, gb_out (cleared by the caller; the
+ * summation order, and so the last bits, vary between runs). */
+int pe_mlp_backward(const pe_mlp_net *net, const void *feat, int rows, const float *const *z,
+                    const void *const *h, const float *dy, void *const *dz, float *const *gw,
+                    float *const *gb, float *gw_out, float *gb_out, void *cuda_stream);
+/* pe_mlp_adam on every parameter (order: weights, biases, w_out, b_out), with
+ * the bf16 weights and their transposes rewritten.  Of `net` the sizes are
+ * read; widths multiples of 32. */
+int pe_mlp_adam_all(const pe_mlp_net *net, float *const *w, const float *const *grad,
+                    float *const *m, float *const *v, void *const *w16, void *const *w16t,
+                    float lr, float beta1, float beta2, float eps, const float *corr,
+                    void *cuda_stream);
+/* out[i] = the network at node first + i of the relative (world) grid, or at
+ * relative state i: features, layers and head in one launch. */
+int pe_mlp_predict_relative_nodes(const pe_mlp_net *net, int64_t first, int64_t n, int positions,
+                                  int headings, int p_speeds, int e_speeds, double extent,
+                                  double p_min, double p_max, double e_min, double e_max,
+                                  float *out, void *cuda_stream);
+int pe_mlp_predict_world_nodes(const pe_mlp_net *net, int64_t first, int64_t n, int positions,
+                               int headings, int p_speeds, int e_speeds, double extent,
+                               double p_min, double p_max, double e_min, double e_max,
+                               float *out, void *cuda_stream);
+int pe_mlp_predict_relative_states(const pe_mlp_net *net, const float *states, int n,
+                                   double extent, double p_min, double p_max, double e_min,
+                                   double e_max, float *out, void *cuda_stream);
+
 /* ------------------------------------------------------------------------
  * Queries of a completed relative table, resident on the GPU.
  *

@@ -15,6 +15,7 @@
 
 #include <cstdint>
 
+#include "mlp_features.cuh"
 #include "pe_internal.h"
 
 namespace pe {
@@ -320,93 +321,54 @@ __global__ void colsum_kernel(const __nv_bfloat16 *x, float *out, int rows, int 
   atomicAdd(out + c, s);
 }
 
-// Relative 5D state [x, y, psi, vP, vE] -> features
-// [x/e, y/e, cos psi, sin psi, vP~, vE~, 0...] (speeds mapped to [-1, 1]),
-// bf16 rows of `ld` elements.
-struct RelFeatureScale {
-  float inv_extent, vp_mid, vp_inv_half, ve_mid, ve_inv_half;
-};
-
-__device__ __forceinline__ void write_rel_features(__nv_bfloat16 *row, int ld,
-                                                   const RelFeatureScale &f, float x,
-                                                   float y, float psi, float vp,
-                                                   float ve) {
-  float s, c;
-  sincosf(psi, &s, &c);
-  const float vals[6] = {x * f.inv_extent, y * f.inv_extent, c, s,
-                         (vp - f.vp_mid) * f.vp_inv_half, (ve - f.ve_mid) * f.ve_inv_half};
-  for (int k = 0; k < ld; k++) row[k] = __float2bfloat16_rn(k < 6 ? vals[k] : 0.f);
+// One feature row of `ld` bf16 elements per row of 16 threads: thread u
+// writes the 16-byte units u, u + 16, ... (the features, then zeros), so that
+// a warp stores two whole rows.  8192 rows of 128: 3 us (40 us when one
+// thread wrote a row element by element).
+template <class Features>
+__device__ __forceinline__ void write_row(__nv_bfloat16 *row, int ld, int u,
+                                          const Features &features) {
+  if (ld % 8 == 0 && ld >= kMaxFeatures && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+    uint4 first = make_uint4(0, 0, 0, 0);
+    if (u < 2) {
+      float v[kMaxFeatures];
+      features(v);
+      first = pack_features(v + 8 * u);
+    }
+    uint4 *out = reinterpret_cast<uint4 *>(row);
+    for (int k = u; k < ld / 8; k += 16) out[k] = k < 2 ? first : make_uint4(0, 0, 0, 0);
+  } else if (u == 0) {
+    float v[kMaxFeatures];
+    features(v);
+    for (int k = 0; k < ld; k++)
+      row[k] = __float2bfloat16_rn(k < kMaxFeatures ? v[k < kMaxFeatures ? k : 0] : 0.f);
+  }
 }
 
-// Grid-node samples of a dense [vP, vE, psi, y, x] table.
-__global__ void encode_relative_nodes_kernel(const float *table, const int64_t *idx,
-                                             int n, int nx, int nh, int nve,
-                                             float extent, float dx, float dphi,
-                                             float vp_lo, float dvp, float ve_lo,
-                                             float dve, RelFeatureScale f,
-                                             __nv_bfloat16 *feat, int ld, float *target) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Grid-node samples of a dense table (WORLD: the 8D one).
+template <bool WORLD>
+__global__ void encode_nodes_kernel(const float *table, const int64_t *idx, int n, NodeGrid g,
+                                    __nv_bfloat16 *feat, int ld, float *target) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, u = threadIdx.x & 15;
   if (i >= n) return;
-  int64_t j = idx[i];
-  const int ix = (int)(j % nx);
-  j /= nx;
-  const int iy = (int)(j % nx);
-  j /= nx;
-  const int ip = (int)(j % nh);
-  j /= nh;
-  const int ie = (int)(j % nve);
-  const int iv = (int)(j / nve);
-  write_rel_features(feat + (int64_t)i * ld, ld, f, fmaf((float)ix, dx, -extent),
-                     fmaf((float)iy, dx, -extent), fmaf((float)ip, dphi, -3.14159265358979f),
-                     fmaf((float)iv, dvp, vp_lo), fmaf((float)ie, dve, ve_lo));
-  if (target) target[i] = table[idx[i]];
+  const int64_t j = idx[i];
+  write_row(feat + (int64_t)i * ld, ld, u, [&](float *v) {
+    if (WORLD)
+      world_node_features(v, g, j);
+    else
+      relative_node_features(v, g, j);
+  });
+  if (target && u == 0) target[i] = table[j];
 }
 
 // Arbitrary relative states [n][5].
-__global__ void encode_relative_states_kernel(const float *states, int n,
-                                              RelFeatureScale f, __nv_bfloat16 *feat,
-                                              int ld) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void encode_relative_states_kernel(const float *states, int n, RelFeatureScale f,
+                                              __nv_bfloat16 *feat, int ld) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, u = threadIdx.x & 15;
   if (i >= n) return;
   const float *s = states + (int64_t)i * 5;
-  write_rel_features(feat + (int64_t)i * ld, ld, f, s[0], s[1], s[2], s[3], s[4]);
-}
-
-// 8D world nodes [xP, yP, thP, vP, xE, yE, thE, vE] -> 10 features.
-__global__ void encode_world_nodes_kernel(const float *table, const int64_t *idx, int n,
-                                          int npos, int nh, int np, int ne, float extent,
-                                          float dx, float dh, float vp_lo, float dvp,
-                                          float ve_lo, float dve, RelFeatureScale f,
-                                          __nv_bfloat16 *feat, int ld, float *target) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int64_t j = idx[i];
-  const int q7 = (int)(j % ne);
-  j /= ne;
-  const int q6 = (int)(j % nh);
-  j /= nh;
-  const int q5 = (int)(j % npos);
-  j /= npos;
-  const int q4 = (int)(j % npos);
-  j /= npos;
-  const int q3 = (int)(j % np);
-  j /= np;
-  const int q2 = (int)(j % nh);
-  j /= nh;
-  const int q1 = (int)(j % npos);
-  const int q0 = (int)(j / npos);
-  float sp, cp, se, ce;
-  sincosf(fmaf((float)q2, dh, -3.14159265358979f), &sp, &cp);
-  sincosf(fmaf((float)q6, dh, -3.14159265358979f), &se, &ce);
-  const float vals[10] = {fmaf((float)q0, dx, -extent) * f.inv_extent,
-                          fmaf((float)q1, dx, -extent) * f.inv_extent, cp, sp,
-                          (fmaf((float)q3, dvp, vp_lo) - f.vp_mid) * f.vp_inv_half,
-                          fmaf((float)q4, dx, -extent) * f.inv_extent,
-                          fmaf((float)q5, dx, -extent) * f.inv_extent, ce, se,
-                          (fmaf((float)q7, dve, ve_lo) - f.ve_mid) * f.ve_inv_half};
-  __nv_bfloat16 *row = feat + (int64_t)i * ld;
-  for (int k = 0; k < ld; k++) row[k] = __float2bfloat16_rn(k < 10 ? vals[k] : 0.f);
-  if (target) target[i] = table[idx[i]];
+  write_row(feat + (int64_t)i * ld, ld, u,
+            [&](float *v) { state_features(v, f, s[0], s[1], s[2], s[3], s[4]); });
 }
 
 }  // namespace
@@ -515,17 +477,6 @@ int pe_mlp_head_backward(const void *h, const float *zprev, const float *w,
   return PE_OK;
 }
 
-static pe::RelFeatureScale feature_scale(float extent, float vp_lo, float vp_hi,
-                                         float ve_lo, float ve_hi) {
-  pe::RelFeatureScale f;
-  f.inv_extent = 1.f / extent;
-  f.vp_mid = 0.5f * (vp_lo + vp_hi);
-  f.vp_inv_half = 2.f / (vp_hi - vp_lo);
-  f.ve_mid = 0.5f * (ve_lo + ve_hi);
-  f.ve_inv_half = 2.f / (ve_hi - ve_lo);
-  return f;
-}
-
 // Features (and table targets when table != NULL) of relative 5D grid nodes
 // given by flat indices into a dense [vP, vE, psi, y, x] table.
 int pe_mlp_encode_relative_nodes(const float *table, const int64_t *idx, int n,
@@ -535,14 +486,9 @@ int pe_mlp_encode_relative_nodes(const float *table, const int64_t *idx, int n,
                                  int ld, float *target, void *cuda_stream) {
   if (!idx || !feat || n <= 0 || ld < 6 || (target && !table))
     return pe::fail(PE_EINVAL, "encode_relative_nodes: invalid arguments");
-  const double pi = 3.14159265358979323846;
-  pe::encode_relative_nodes_kernel<<<(n + 255) / 256, 256, 0,
-                                     static_cast<cudaStream_t>(cuda_stream)>>>(
-      table, idx, n, positions, headings, e_speeds, (float)extent,
-      (float)(2 * extent / (positions - 1)), (float)(2 * pi / headings), (float)p_min,
-      (float)((p_max - p_min) / (p_speeds - 1)), (float)e_min,
-      (float)((e_max - e_min) / (e_speeds - 1)),
-      feature_scale((float)extent, (float)p_min, (float)p_max, (float)e_min, (float)e_max),
+  pe::encode_nodes_kernel<false><<<(n + 15) / 16, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+      table, idx, n,
+      pe::node_grid(positions, headings, p_speeds, e_speeds, extent, p_min, p_max, e_min, e_max),
       static_cast<__nv_bfloat16 *>(feat), ld, target);
   PE_CUDA_TRY(cudaGetLastError());
   pe::count_launches(1);
@@ -555,10 +501,10 @@ int pe_mlp_encode_relative_states(const float *states, int n, double extent,
                                   double e_max, void *feat, int ld, void *cuda_stream) {
   if (!states || !feat || n <= 0 || ld < 6)
     return pe::fail(PE_EINVAL, "encode_relative_states: invalid arguments");
-  pe::encode_relative_states_kernel<<<(n + 255) / 256, 256, 0,
+  pe::encode_relative_states_kernel<<<(n + 15) / 16, 256, 0,
                                       static_cast<cudaStream_t>(cuda_stream)>>>(
       states, n,
-      feature_scale((float)extent, (float)p_min, (float)p_max, (float)e_min, (float)e_max),
+      pe::feature_scale((float)extent, (float)p_min, (float)p_max, (float)e_min, (float)e_max),
       static_cast<__nv_bfloat16 *>(feat), ld);
   PE_CUDA_TRY(cudaGetLastError());
   pe::count_launches(1);
@@ -574,14 +520,9 @@ int pe_mlp_encode_world_nodes(const float *table, const int64_t *idx, int n,
                               void *cuda_stream) {
   if (!idx || !feat || n <= 0 || ld < 10 || (target && !table))
     return pe::fail(PE_EINVAL, "encode_world_nodes: invalid arguments");
-  const double pi = 3.14159265358979323846;
-  pe::encode_world_nodes_kernel<<<(n + 255) / 256, 256, 0,
-                                  static_cast<cudaStream_t>(cuda_stream)>>>(
-      table, idx, n, positions, headings, p_speeds, e_speeds, (float)extent,
-      (float)(2 * extent / (positions - 1)), (float)(2 * pi / headings), (float)p_min,
-      (float)((p_max - p_min) / (p_speeds - 1)), (float)e_min,
-      (float)((e_max - e_min) / (e_speeds - 1)),
-      feature_scale((float)extent, (float)p_min, (float)p_max, (float)e_min, (float)e_max),
+  pe::encode_nodes_kernel<true><<<(n + 15) / 16, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+      table, idx, n,
+      pe::node_grid(positions, headings, p_speeds, e_speeds, extent, p_min, p_max, e_min, e_max),
       static_cast<__nv_bfloat16 *>(feat), ld, target);
   PE_CUDA_TRY(cudaGetLastError());
   pe::count_launches(1);

@@ -21,81 +21,15 @@
 // warps run the epilogue, warp w on accumulator lanes 32w..32w+31 (= tile
 // rows).  Every mbarrier wait is bounded; a timed-out wait sets the
 // error flag and the CTA still releases its tensor memory.
-#include <cuda.h>
-#include <cuda_bf16.h>
-
-#include "pe_internal.h"
+#include "mlp_tc.cuh"
 
 namespace pe {
 namespace {
 
-constexpr int TM = 128, TK = 64, STAGES = 2, THREADS = 128;
+using namespace tc;
+
+constexpr int STAGES = 2, THREADS = 128;
 constexpr int A_BYTES = TM * TK * 2;  // 16 KB
-constexpr uint32_t WAIT_LIMIT = 1u << 24;
-
-__device__ __forceinline__ float silu(float z) { return z / (1.f + __expf(-z)); }
-__device__ __forceinline__ float silu_grad(float z) {
-  const float s = 1.f / (1.f + __expf(-z));
-  return s * (1.f + z * (1.f - s));
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile(
-      "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-      "r"(bytes)
-      : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n"
-      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait on a phase; false (and the error flag set) on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, unsigned *error) {
-  for (uint32_t i = 0; i < WAIT_LIMIT; i++)
-    if (mbar_try_wait(bar, parity)) return true;
-  atomicOr(error, 1u);
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y,
-                                            uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major, 128B-swizzled operand tile
-// (rows of 128 bytes, 8-row groups 1024 bytes apart): start address and
-// offsets in 16-byte units, descriptor version 1, swizzle mode 128B.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFF) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                  // leading byte offset (unused when swizzled)
-  d |= (uint64_t)(1024 >> 4) << 32;        // stride byte offset: next 8-row group
-  d |= (uint64_t)1 << 46;                  // descriptor version
-  d |= (uint64_t)2 << 61;                  // 128-byte swizzle
-  return d;
-}
 
 // Instruction descriptor: BF16 x BF16 -> FP32, both K-major, M = 128, N = TN.
 template <int TN>
@@ -114,13 +48,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t 
       " setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
       "l"(da), "l"(db), "r"(idesc<TN>()), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
       : "memory");
 }
 
@@ -280,48 +207,19 @@ __host__ __device__ constexpr size_t smem_bytes() {
   return 1024 + STAGES * (A_BYTES + TN * TK * 2) + (2 * STAGES + 1) * 8 + 16;
 }
 
-// 2D tensor map of a K-major bf16 matrix [rows][K] with row pitch ld
-// elements, box 64 (K) x box_rows, 128-byte swizzle.
-// The driver's tensor-map encoder, fetched through the runtime so that the
-// library does not link libcuda (it loads on machines without a driver).
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                 const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+}  // namespace
 
-EncodeTiled encoder() {
-  static EncodeTiled fn = nullptr;
-  if (!fn) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiled>(p);
-  }
-  return fn;
-}
-
-CUresult make_map(CUtensorMap *map, const void *ptr, int rows, int K, int ld, int box_rows) {
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {TK, (cuuint32_t)box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  EncodeTiled encode = encoder();
-  if (!encode) return CUDA_ERROR_NOT_FOUND;
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                                const_cast<void *>(ptr), dims, strides, box, elem,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-}
-
+namespace tc {
 unsigned *error_word() {
   static unsigned *word = nullptr;  // one per process (first device used)
   if (!word && cudaMalloc(&word, sizeof(unsigned)) == cudaSuccess)
     cudaMemset(word, 0, sizeof(unsigned));
   return word;
 }
+
+}  // namespace tc
+
+namespace {
 
 template <int EPI, int TN>
 cudaError_t launch(const CUtensorMap &a, const CUtensorMap &b, const TcArgs &g,
@@ -352,6 +250,7 @@ int pe_mlp_gemm_tc(const void *A, const void *B, int M, int N, int K, int lda, i
                    int epilogue, float *C32, void *C16, int ldc, const float *bias,
                    const float *zpre, void *cuda_stream) {
   using namespace pe;
+  using namespace pe::tc;
   if (!A || !B || M <= 0 || N <= 0 || K <= 0 || M % TM || N % 128 || K % TK)
     return fail(PE_EINVAL, "gemm_tc: M, N multiples of 128, K a multiple of 64");
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) % 16 || lda % 8 ||
@@ -385,6 +284,7 @@ int pe_mlp_gemm_tc(const void *A, const void *B, int M, int N, int K, int lda, i
 int pe_mlp_gemm_tc_splitk(const void *A, const void *B, int M, int N, int K, int lda, int ldb,
                           int splits, float *C32, int ldc, void *cuda_stream) {
   using namespace pe;
+  using namespace pe::tc;
   if (!A || !B || !C32 || M <= 0 || N <= 0 || K <= 0 || splits < 1 || M % TM || N % 128 ||
       K % (TK * splits))
     return fail(PE_EINVAL,
@@ -411,6 +311,7 @@ int pe_mlp_gemm_tc_splitk(const void *A, const void *B, int M, int N, int K, int
 // clear the flag).  Synchronises the device.
 int pe_mlp_gemm_tc_timeouts(int32_t *count) {
   using namespace pe;
+  using namespace pe::tc;
   if (!count) return fail(PE_EINVAL, "count is NULL");
   unsigned *w = error_word(), h = 0;
   if (!w) return fail(PE_ENOMEM, "gemm_tc: error word");

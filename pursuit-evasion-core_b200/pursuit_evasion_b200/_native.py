@@ -168,6 +168,14 @@ class VehicleModel(ctypes.Structure):
 
 
 # name -> (restype, argtypes)
+class MlpNet(ctypes.Structure):
+    """pe_mlp_net: the surrogate's sizes and parameter pointers."""
+    _fields_ = [("layers", ctypes.c_int32), ("hidden", ctypes.c_int32),
+                ("in_width", ctypes.c_int32), ("w16", ctypes.c_void_p * 8),
+                ("w16t", ctypes.c_void_p * 8), ("b", ctypes.c_void_p * 8),
+                ("w_out", ctypes.c_void_p), ("b_out", ctypes.c_void_p)]
+
+
 SIGNATURES = {
     "pe_version": (ctypes.c_int, []),
     "pe_last_error": (ctypes.c_char_p, []),
@@ -364,6 +372,18 @@ SIGNATURES = {
                                       + [_P, ctypes.c_int, _P]),
     "pe_mlp_encode_world_nodes": (ctypes.c_int, [_P, _P] + [ctypes.c_int] * 5
                                   + [ctypes.c_double] * 5 + [_P, ctypes.c_int, _P, _P]),
+    "pe_mlp_forward": (ctypes.c_int, [ctypes.POINTER(MlpNet), _P, ctypes.c_int] + [_P] * 7),
+    "pe_mlp_backward": (ctypes.c_int, [ctypes.POINTER(MlpNet), _P, ctypes.c_int] + [_P] * 9),
+    "pe_mlp_adam_all": (ctypes.c_int, [ctypes.POINTER(MlpNet)] + [_P] * 6
+                        + [ctypes.c_float] * 4 + [_P, _P]),
+    "pe_mlp_predict_relative_nodes": (ctypes.c_int, [ctypes.POINTER(MlpNet), ctypes.c_int64,
+                                                     ctypes.c_int64] + [ctypes.c_int] * 4
+                                      + [ctypes.c_double] * 5 + [_P, _P]),
+    "pe_mlp_predict_world_nodes": (ctypes.c_int, [ctypes.POINTER(MlpNet), ctypes.c_int64,
+                                                  ctypes.c_int64] + [ctypes.c_int] * 4
+                                   + [ctypes.c_double] * 5 + [_P, _P]),
+    "pe_mlp_predict_relative_states": (ctypes.c_int, [ctypes.POINTER(MlpNet), _P, ctypes.c_int]
+                                       + [ctypes.c_double] * 5 + [_P, _P]),
 }
 
 _lib = None

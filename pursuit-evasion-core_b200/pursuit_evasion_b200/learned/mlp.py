@@ -5,12 +5,13 @@ Architecture (BF16 weights and activations, FP32 accumulation):
 The features of a relative 5D state [x, y, psi, vP, vE] are
 [x/e, y/e, cos psi, sin psi, vP~, vE~] (speeds mapped to [-1, 1]); of an 8D
 state, the same per car.  Every forward, backward and Adam kernel is
-hand-written (csrc/mlp.cu, csrc/mlp_tc.cu, C ABI pe_mlp_*): the layer and
-activation-gradient GEMMs run on the tensor cores with tcgen05.mma and the
-accumulator in tensor memory, the split-K weight-gradient GEMM on mma.sync,
-which reads the row-major activations as they are (the tcgen05 split-K
-product, pe_mlp_gemm_tc_splitk, is faster alone but needs both operands
-transposed first, and the transposes cost more than it saves).
+hand-written (C ABI pe_mlp_*).  Networks of the default width run as whole-
+network kernels on the tensor cores (csrc/mlp_fused.cu): forward with the
+head, backward of the activations with the bias and head gradients, every
+weight gradient, and Adam, one launch each; inference makes its features in
+the same launch.  Other widths take a launch per layer (csrc/mlp_tc.cu,
+csrc/mlp.cu): layer and activation-gradient GEMMs on tcgen05.mma, the split-K
+weight-gradient GEMM on mma.sync.
 PyTorch only provides device memory, the stream, random numbers for
 minibatches and, in the tests, the FP64 autograd that checks the gradients.  The reference's precedent is a
 SiLU MLP trained with Adam on MSE against DP labels
@@ -33,6 +34,11 @@ LAYERS = 4
 
 def _ptr(t):
     return ctypes.c_void_p(t.data_ptr())
+
+
+def _ptrs(tensors):
+    """A C array of the tensors' device pointers."""
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
 class ValueMLP:
@@ -71,7 +77,12 @@ class ValueMLP:
         self.params = self.w + self.b + [self.w_out, self.b_out]
         self.m = [torch.zeros_like(p) for p in self.params]
         self.v = [torch.zeros_like(p) for p in self.params]
-        self.grads = [torch.zeros_like(p) for p in self.params]
+        # gradients: views of one buffer, cleared in one launch
+        self._grad_flat = torch.zeros(sum(p.numel() for p in self.params), device=self.dev)
+        self.grads, at = [], 0
+        for p in self.params:
+            self.grads.append(self._grad_flat[at:at + p.numel()].view_as(p))
+            at += p.numel()
         self.corr = torch.ones(2, device=self.dev)
         self.loss = torch.zeros(1, device=self.dev)
         self._alloc(max_batch)
@@ -94,6 +105,21 @@ class ValueMLP:
         """Reallocate the activation buffers for `batch` rows (for instance
         large inference chunks after training); weights are kept."""
         self._alloc(int(batch))
+
+    @property
+    def fused(self):
+        """Whether the whole-network kernels take this network."""
+        return self.hidden == 256 and 1 <= self.layers <= 8
+
+    def native_net(self):
+        """The parameters as the C ABI's pe_mlp_net."""
+        net = _native.MlpNet(self.layers, self.hidden, FEATURES)
+        for l in range(self.layers):
+            net.w16[l] = self.w16[l].data_ptr()
+            net.w16t[l] = self.w16t[l].data_ptr()
+            net.b[l] = self.b[l].data_ptr()
+        net.w_out, net.b_out = self.w_out.data_ptr(), self.b_out.data_ptr()
+        return net
 
     # ----------------------------------------------------------- kernels
     def _stream(self):
@@ -123,6 +149,13 @@ class ValueMLP:
         """Forward over self.feat[:rows]; with target=True also the MSE loss
         (accumulated into self.loss) and dy.  inference=True skips storing
         the FP32 pre-activations, which only backward() reads."""
+        if self.fused:
+            opt = lambda t: _ptr(t) if target else None
+            _native.check(self.lib.pe_mlp_forward(
+                ctypes.byref(self.native_net()), _ptr(self.feat), rows,
+                None if inference else _ptrs(self.z), _ptrs(self.h), opt(self.target),
+                _ptr(self.y), opt(self.dy), opt(self.loss), self._stream()))
+            return self.y[:rows]
         x = self.feat
         for l in range(self.layers):
             K = FEATURES if l == 0 else self.hidden
@@ -139,11 +172,16 @@ class ValueMLP:
 
     def backward(self, rows):
         """Gradients of the MSE of the last forward(target=True) into self.grads."""
-        for g in self.grads:
-            g.zero_()
+        self._grad_flat.zero_()
         L = self.layers
         gw, gb = self.grads[:L], self.grads[L:2 * L]
         gw_out, gb_out = self.grads[2 * L], self.grads[2 * L + 1]
+        if self.fused:
+            _native.check(self.lib.pe_mlp_backward(
+                ctypes.byref(self.native_net()), _ptr(self.feat), rows, _ptrs(self.z),
+                _ptrs(self.h), _ptr(self.dy), _ptrs(self.dz), _ptrs(gw), _ptrs(gb),
+                _ptr(gw_out), _ptr(gb_out), self._stream()))
+            return
         _native.check(self.lib.pe_mlp_head_backward(
             _ptr(self.h[-1]), _ptr(self.z[-1]), _ptr(self.w_out), _ptr(self.dy),
             _ptr(gw_out), _ptr(gb_out), _ptr(self.dz[-1]), rows, self.hidden,
@@ -167,6 +205,12 @@ class ValueMLP:
     def adam(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8):
         """One Adam update; the bias corrections are read from self.corr on
         the device (set them with set_step before the call or graph replay)."""
+        if self.fused:
+            _native.check(self.lib.pe_mlp_adam_all(
+                ctypes.byref(self.native_net()), _ptrs(self.params), _ptrs(self.grads),
+                _ptrs(self.m), _ptrs(self.v), _ptrs(self.w16), _ptrs(self.w16t), lr, beta1,
+                beta2, eps, _ptr(self.corr), self._stream()))
+            return
         for i, (p, g, m, v) in enumerate(zip(self.params, self.grads, self.m, self.v)):
             w16 = _ptr(self.w16[i]) if i < self.layers else None
             _native.check(self.lib.pe_mlp_adam(_ptr(p), w16, _ptr(g), _ptr(m), _ptr(v),

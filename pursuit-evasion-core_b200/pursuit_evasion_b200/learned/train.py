@@ -40,6 +40,12 @@ class RelativeNodeSampler:
             _ptr(net.feat), FEATURES, _ptr(net.target) if with_target else None,
             net._stream()))
 
+    def predict(self, net, first, rows, out):
+        """Network values of the nodes first .. first + rows - 1 into the
+        contiguous float32 device tensor `out` (networks with net.fused)."""
+        _native.check(_native.library().pe_mlp_predict_relative_nodes(
+            ctypes.byref(net.native_net()), first, rows, *self.args, _ptr(out), net._stream()))
+
 
 class WorldNodeSampler:
     """8D grid nodes [xP, yP, thP, vP, xE, yE, thE, vE] of a dense table."""
@@ -61,6 +67,12 @@ class WorldNodeSampler:
             _ptr(self.table) if with_target else None, _ptr(idx), rows, *self.args,
             _ptr(net.feat), FEATURES, _ptr(net.target) if with_target else None,
             net._stream()))
+
+    def predict(self, net, first, rows, out):
+        """Network values of the nodes first .. first + rows - 1 into the
+        contiguous float32 device tensor `out` (networks with net.fused)."""
+        _native.check(_native.library().pe_mlp_predict_world_nodes(
+            ctypes.byref(net.native_net()), first, rows, *self.args, _ptr(out), net._stream()))
 
 
 def train(net, sampler, *, samples=1 << 22, epochs=20, batch=8192, lr=1e-3,
@@ -118,6 +130,17 @@ def predict_nodes(net, sampler, out, *, chunk=8192):
     torch = net.torch
     dev = net.dev
     n = sampler.cells
+    if net.fused and chunk > 0 and n > 0 and hasattr(sampler, "predict"):
+        direct = (out.dtype == torch.float32 and out.is_contiguous()
+                  and out.device == dev and out.dim() == 1 and out.numel() >= n)
+        values = out if direct else torch.empty(n, dtype=torch.float32, device=dev)
+        step = 1 << 30  # rows of one launch
+        for start in range(0, n, step):
+            rows = min(step, n - start)
+            sampler.predict(net, start, rows, values[start:start + rows])
+        if not direct:
+            out[:n].copy_(values)
+        return out
     chunk = min(chunk, net.batch)
     idx = torch.empty(chunk, dtype=torch.int64, device=dev)
     for start in range(0, n, chunk):
@@ -140,6 +163,13 @@ def predict_states(net, config, extent, states):
         raise ValueError("query batch exceeds the network's buffers")
     p, e = config.pursuer, config.evader
     lib = _native.library()
+    if net.fused:
+        out = torch.empty(n, dtype=torch.float32, device=net.dev)
+        _native.check(lib.pe_mlp_predict_relative_states(
+            ctypes.byref(net.native_net()), _ptr(states), n, float(extent), float(p.speed_min),
+            float(p.speed_max), float(e.speed_min), float(e.speed_max), _ptr(out),
+            net._stream()))
+        return out
     _native.check(lib.pe_mlp_encode_relative_states(
         _ptr(states), n, float(extent), float(p.speed_min), float(p.speed_max),
         float(e.speed_min), float(e.speed_max), _ptr(net.feat), FEATURES, net._stream()))
