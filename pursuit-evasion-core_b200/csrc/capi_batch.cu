@@ -23,6 +23,7 @@ struct pe_batch {
   int count = 0;
   int device = 0;
   bool exact = true;
+  bool tiled = true;  // the tiled kernels; else (exact) a cell per thread
   std::vector<pe_relative_params> params;  // caller's order
   std::vector<double> horizons;
   std::vector<pe::Rel5Grid> grids;
@@ -48,7 +49,7 @@ struct pe_batch {
   cudaGraphExec_t graph = nullptr;
   cudaStream_t graph_stream = nullptr;
   int grid = 0;
-  size_t tiled_smem = 0;  // dynamic shared memory of the tiled float32 kernel
+  size_t tiled_smem = 0;  // dynamic shared memory of the tiled kernel
   bool initialized = false;
   pe::LaunchTimer timer;
 };
@@ -84,11 +85,46 @@ int check_solve(const pe_batch *h, int32_t solve) {
   return PE_OK;
 }
 
+// Headings per item of the tiled exact kernel: the cap (all headings, or 24,
+// 16, 12, 8, 6) of least estimated time.  A stage's time is its items' heading
+// steps over the CTAs -- an item also pays about 3 steps to start -- plus half
+// an item for the CTAs that end last: few solves want short items, a full
+// batch whole stacks.
+int exact_chunk_cap(const pe_batch *h, int ctas) {
+  int best = 1 << 20;
+  double best_time = 1e300;
+  for (int cap : {1 << 20, 24, 16, 12, 8, 6}) {
+    std::vector<double> work(h->count), longest(h->count);
+    for (int pos = 0; pos < h->count; pos++) {
+      const int i = h->order[pos];
+      const pe::Rel5Grid &g = h->grids[i];
+      const int rows = pe::rel5_batch_tiled_rows(g.nx, g.xp, h->rows[i]);
+      const int chunks = (g.nh + cap - 1) / cap, chunk = (g.nh + chunks - 1) / chunks;
+      const double item = chunk + 3, warps = (rows * (g.xp / 4) + 31) / 32;
+      work[pos] = (pos ? work[pos - 1] : 0) + item * warps * chunks * g.nvp * g.nve *
+                                                  ((g.nx + rows - 1) / rows);
+      longest[pos] = std::max(pos ? longest[pos - 1] : 0.0, item * warps);
+    }
+    double time = 0;  // solves still stepping at step k are a prefix
+    for (int pos = h->count - 1; pos >= 0; pos--) {
+      const size_t after = pos + 1 < h->count ? h->steps[h->order[pos + 1]].size() : 0;
+      time += (double)(h->steps[h->order[pos]].size() - after) *
+              (work[pos] / ctas + 0.5 * longest[pos]);
+    }
+    if (time < best_time * 0.999) {
+      best_time = time;
+      best = cap;
+    }
+  }
+  return best;
+}
+
 // Descriptors and the active-item prefix for the current tiles.
 int upload_descriptors(pe_batch *h) {
   std::vector<pe::Rel5BatchSolve> d(h->count);
   int64_t base = 0;
   size_t smem = 0;
+  const int cap = h->exact && h->tiled ? exact_chunk_cap(h, 2 * 148) : 1 << 20;
   for (int pos = 0; pos < h->count; pos++) {
     const int i = h->order[pos];
     const pe::Rel5Grid &g = h->grids[i];
@@ -102,24 +138,28 @@ int upload_descriptors(pe_batch *h) {
     s.steps = h->step_table + h->step_off[i];
     s.stats = h->stats + i;
     s.nsteps = (int)h->steps[i].size();
-    if (h->exact) {
+    const int chunks = (g.nh + cap - 1) / cap;
+    s.chunk = (g.nh + chunks - 1) / chunks;
+    if (!h->tiled) {
       // item: `rows` y rows of one (vP, vE, psi) plane
       s.rows = h->rows[i];
       s.items = (int64_t)g.nvp * g.nve * g.nh * ((g.nx + s.rows - 1) / s.rows);
     } else {
       // item: `rows` y rows of one (vP, vE) plane stack, all headings
+      // (float32) or a chunk of them (exact)
       s.rows = pe::rel5_batch_tiled_rows(g.nx, g.xp, h->rows[i]);
-      s.items = (int64_t)g.nvp * g.nve * ((g.nx + s.rows - 1) / s.rows);
+      s.items = (int64_t)g.nvp * g.nve * ((g.nx + s.rows - 1) / s.rows) *
+                (h->exact ? (g.nh + s.chunk - 1) / s.chunk : 1);
       smem = std::max(smem, pe::rel5_batch_tiled_smem(s.rows, g.xp));
     }
     s.item_base = base;
     base += s.items;
   }
-  if (!h->exact && smem != h->tiled_smem) {
+  if (h->tiled && smem != h->tiled_smem) {
     // a different launch shape: size the cooperative grid again and record
     // a new graph at the next run
     h->tiled_smem = smem;
-    h->grid = pe::rel5_batch_grid_tiled(smem);
+    h->grid = h->exact ? pe::rel5_batch_grid_tiled_exact(smem) : pe::rel5_batch_grid_tiled(smem);
     if (h->grid <= 0) return fail(PE_EINVAL, "batch tiles do not fit the tiled kernel");
     if (h->graph) {
       cudaGraphExecDestroy(h->graph);
@@ -158,8 +198,10 @@ int capture(pe_batch *h) {
   PE_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaMemsetAsync(h->sync, 0, 4 * sizeof(unsigned), h->stream);
   if (err == cudaSuccess)
-    err = h->exact ? pe::rel5_batch_run_exact(args, h->grid, h->stream)
-                   : pe::rel5_batch_run_tiled(args, h->grid, h->tiled_smem, h->stream);
+    err = !h->tiled ? pe::rel5_batch_run_exact(args, h->grid, h->stream)
+          : h->exact
+              ? pe::rel5_batch_run_tiled_exact(args, h->grid, h->tiled_smem, h->stream)
+              : pe::rel5_batch_run_tiled(args, h->grid, h->tiled_smem, h->stream);
   cudaError_t end = cudaStreamEndCapture(h->stream, &g);
   if (err == cudaSuccess) err = end;
   if (err == cudaSuccess) err = cudaGraphInstantiate(&h->graph, g, 0);
@@ -228,10 +270,13 @@ int pe_batch_create(const pe_relative_params *params, const double *horizons, in
     }
     h->max_steps = std::max(h->max_steps, (int)st.size());
     h->steps.push_back(std::move(st));
-    // default tile: about one cell per thread (exact), the widest item the
-    // CTA holds (tiled float32)
-    h->rows.push_back(h->exact ? std::max(1, std::min(g.nx, (256 + g.nx - 1) / g.nx))
-                               : pe::rel5_batch_tiled_rows(g.nx, g.xp, 0));
+    // default tile: the widest item the CTA holds (float32), that many rows
+    // spread evenly over the slabs (exact)
+    const int widest = pe::rel5_batch_tiled_rows(g.nx, g.xp, 0);
+    const int slabs = (g.nx + widest - 1) / widest;
+    h->rows.push_back(h->exact ? (g.nx + slabs - 1) / slabs : widest);
+    // rows wider than a CTA's threads take a cell per thread
+    if (h->exact && g.xp / 4 > pe::kRel5BatchThreads) h->tiled = false;
     h->field_off.push_back(fields);
     fields += 3 * (size_t)g.n_padded;
     h->table_off.push_back(tables);
@@ -284,7 +329,7 @@ int pe_batch_create(const pe_relative_params *params, const double *horizons, in
     take(cudaMemset(h->sync, 0, 4 * sizeof(unsigned)));
   }
   if (err == cudaSuccess) {
-    if (h->exact) {  // the tiled kernel's grid is sized with its tiles
+    if (!h->tiled) {  // a tiled kernel's grid is sized with its tiles
       h->grid = pe::rel5_batch_grid_exact();
       if (h->grid <= 0) err = cudaErrorInvalidConfiguration;
     }

@@ -19,7 +19,8 @@ struct Rel5BatchSolve {
   Rel5Stats *stats;        // residual of the last step, largest increase, flags
   int nsteps;
   int rows;                // y rows per work item (the tile)
-  int64_t items;           // work items of one stage: nvp * nve * nh * ceil(nx / rows)
+  int chunk;               // headings per work item (tiled exact kernel)
+  int64_t items;           // work items of one stage
   int64_t item_base;       // index of the solve's first item in the batch
 };
 
@@ -42,6 +43,13 @@ int rel5_batch_grid_exact();
 // sync[2]).  `sync` must be zeroed before the launch.  Exact: the
 // single-grid exact path's arithmetic (each solve equals it bit for bit).
 cudaError_t rel5_batch_run_exact(const Rel5BatchArgs &args, int grid, cudaStream_t stream);
+
+// The same, tiled (relative5d_batch_tiled_exact.cu): a work item is `rows` y
+// rows of one (vP, vE) plane stack over `chunk` headings; rows and smem as for
+// the tiled float32 kernel below.
+int rel5_batch_grid_tiled_exact(size_t smem);
+cudaError_t rel5_batch_run_tiled_exact(const Rel5BatchArgs &args, int grid, size_t smem,
+                                       cudaStream_t stream);
 
 // Float32 update, tiled (relative5d_batch_tiled.cu): a work item is `rows` y
 // rows of one (vP, vE) plane stack, all headings, one thread per 4-cell x

@@ -129,12 +129,35 @@ struct HeadingCarry {
   }
 };
 
-// Per-item constants of the update (all uniform over the item's cells of one
-// row).
+// Constants of an item (uniform over its threads; may lie in shared memory).
 struct ItemCoef {
-  double y, vp, ve, wp, we, acc_p, acc_e, dt;
-  int iv, nvp, ie, nve, iy, nx;
-  bool y_general, v_general, e_general;
+  double vp, ve, wp, we, acc_p, acc_e, dt;
+  int iv, nvp, ie, nve, nx;
+  bool v_general, e_general;
+
+  __device__ __forceinline__ void set(const Rel5Grid &g, int iv_, int ie_, double dt_) {
+    iv = iv_;
+    nvp = g.nvp;
+    ie = ie_;
+    nve = g.nve;
+    nx = g.nx;
+    v_general = iv < 2 || iv + 2 >= g.nvp;
+    e_general = ie < 2 || ie + 2 >= g.nve;
+    vp = g.vp_lo + iv * g.dvp;
+    ve = g.ve_lo + ie * g.dve;
+    wp = fabs(vp) * g.curv_p;
+    we = fabs(ve) * g.curv_e;
+    acc_p = g.acc_p;
+    acc_e = g.acc_e;
+    dt = dt_;
+  }
+};
+
+// A thread's row: its y, and whether its warp takes the general y rules.
+struct RowCoef {
+  double y;
+  int iy;
+  bool general;
 };
 
 struct AxisSteps {
@@ -142,18 +165,19 @@ struct AxisSteps {
 };
 
 // The 4 cells' Hamiltonian plus dissipation at heading k.  w: the row window
-// x0-2 .. x0+5 (w[2..5] the cells); ym2..yp2 the rows iy-2 .. iy+2; em2..ep2
-// and vm2..vp2 the speed neighbours; VN, VNEW headings k+1, k+2.  XR = nx mod
-// 4 places the x end rules: node nx-2 sits at cell KP of its chunk, node nx-1
-// at cell IEND; the flags say whether this chunk holds x = 0, node nx-2, node
-// nx-1.
+// x0-2 .. x0+5 (C the cells); ycol the chunk's column in the own rows (rows
+// iy-2 .. iy+2 ystride apart), nb in the speed-neighbour rows (vE-2, -1, +1, +2,
+// vP-2 .. nbstride apart); VN, VNEW headings k+1, k+2.  XR = nx mod 4 places the
+// x end rules at compile time, `kend` and `iend` saying whether nodes nx-2 and
+// nx-1 lie in this chunk; XR = -1 takes their cells from `kcell` and `icell`
+// (outside 0..3 where the chunk does not hold them).
 template <int ORDER, int XR>
 __device__ __forceinline__ void walk_hamiltonian(
     const float2 &xl, const float4 &C, const float2 &xr, const float4 &VN, const float4 &VNEW,
     const float *ycol, int ystride, const float *nb, int nbstride, bool first, bool kend,
-    bool iend, const double *xs, double cs, double sn, const ItemCoef &q, const AxisSteps &st,
+    bool iend, int kcell, int icell, const double *xs, double cs, double sn, const ItemCoef &q,
+    const RowCoef &row, const AxisSteps &st,
     HeadingCarry<ORDER> &carry, double H[4]) {
-  constexpr int KP = (XR + 2) & 3, IEND = (XR + 3) & 3;
   const double bx = q.ve * cs - q.vp, by = q.ve * sn;
   double gx[4], gy[4], diss[4];
   {
@@ -166,11 +190,13 @@ __device__ __forceinline__ void walk_hamiltonian(
 #pragma unroll
       for (int i = 0; i < 6; i++) c2[i] = quot2(w[i + 2], w[i + 1], w[i], st.x);
       c2[1] = first ? c2[2] : c2[1];
-      c2[KP + 2] = kend ? c2[KP + 1] : c2[KP + 2];
+#pragma unroll
+      for (int i = 3; i >= 0; i--)
+        if (XR < 0 || i == ((XR + 2) & 3)) c2[i + 2] = (XR < 0 ? kcell == i : kend) ? c2[i + 1] : c2[i + 2];
 #pragma unroll
       for (int i = 0; i < 5; i++) E[i] = edge_term(c2[i], c2[i + 1], st.x);
     }
-    const double ax = fabs(bx) + q.wp * fabs(q.y);
+    const double ax = fabs(bx) + q.wp * fabs(row.y);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       double lo = ORDER == 2 ? D[i] + E[i] : D[i];
@@ -179,9 +205,10 @@ __device__ __forceinline__ void walk_hamiltonian(
         lo = first ? D[1] : lo;
         hi = first ? D[1] : hi;
       }
-      if (i == IEND) {
-        lo = iend ? D[i] : lo;
-        hi = iend ? D[i] : hi;
+      if (XR < 0 || i == ((XR + 3) & 3)) {
+        const bool at_end = XR < 0 ? icell == i : iend;
+        lo = at_end ? D[i] : lo;
+        hi = at_end ? D[i] : hi;
       }
       gx[i] = .5 * (lo + hi);
       diss[i] = ax * (hi - lo);
@@ -197,10 +224,10 @@ __device__ __forceinline__ void walk_hamiltonian(
     for (int i = 0; i < 4; i++) {
       const double v = f4_get(C, i);
       const Slopes s =
-          q.y_general ? axis_slopes<ORDER, true>(f4_get(m2, i), f4_get(m1, i), v, f4_get(p1, i),
-                                                 f4_get(p2, i), q.iy, q.nx, st.x)
+          row.general ? axis_slopes<ORDER, true>(f4_get(m2, i), f4_get(m1, i), v, f4_get(p1, i),
+                                                 f4_get(p2, i), row.iy, q.nx, st.x)
                       : axis_slopes<ORDER, false>(f4_get(m2, i), f4_get(m1, i), v,
-                                                  f4_get(p1, i), f4_get(p2, i), q.iy, q.nx, st.x);
+                                                  f4_get(p1, i), f4_get(p2, i), row.iy, q.nx, st.x);
       gy[i] = .5 * (s.lo + s.hi);
       diss[i] = diss[i] + (aby + q.wp * fabs(xs[i])) * (s.hi - s.lo);
     }
@@ -211,7 +238,7 @@ __device__ __forceinline__ void walk_hamiltonian(
     const Slopes s = carry.next(i, (double)f4_get(C, i), f4_get(VN, i), f4_get(VNEW, i), st.psi);
     const double gp = .5 * (s.lo + s.hi);
     diss[i] = diss[i] + ap * (s.hi - s.lo);
-    H[i] = bx * gx[i] + by * gy[i] - q.wp * fabs(q.y * gx[i] - xs[i] * gy[i] - gp) +
+    H[i] = bx * gx[i] + by * gy[i] - q.wp * fabs(row.y * gx[i] - xs[i] * gy[i] - gp) +
            q.we * fabs(gp);
   }
   double je[4];  // the evader axis' jump: its slopes come first in the dissipation's
@@ -324,7 +351,7 @@ __device__ __noinline__ bool slow_cell(const Rel5Grid &g, const Rel5Stage &s, in
 template <int ORDER, int BLEND>
 __device__ __forceinline__ bool walk_update(const Rel5Grid &g, const Rel5Stage &s, int x0,
                                             int ip, int64_t j, int valid, const ItemCoef &q,
-                                            const double *xs, const float4 &C,
+                                            const RowCoef &row, const double *xs, const float4 &C,
                                             const float4 &P, const double H[4],
                                             ChangeMax &change) {
   float now[4], prev[4];
@@ -340,7 +367,7 @@ __device__ __forceinline__ bool walk_update(const Rel5Grid &g, const Rel5Stage &
     redo |= !ok && i < valid;
   }
   if (s.exit_r2 > 0) {
-    const double yy = q.y * q.y;
+    const double yy = row.y * row.y;
 #pragma unroll
     for (int i = 0; i < 4; i++)
       if (xs[i] * xs[i] + yy > s.exit_r2) now[i] = prev[i] = (float)s.exit_r;
@@ -348,7 +375,7 @@ __device__ __forceinline__ bool walk_update(const Rel5Grid &g, const Rel5Stage &
   bool bad = false;
   if (redo) {  // every cell of the chunk, in the general form
     for (int i = 0; i < valid; i++)
-      bad |= slow_cell<ORDER, BLEND>(g, s, x0 + i, q.iy, ip, q.iv, q.ie, j + i,
+      bad |= slow_cell<ORDER, BLEND>(g, s, x0 + i, row.iy, ip, q.iv, q.ie, j + i,
                                      &change.abs_max, &change.up_max);
     return bad;
   }

@@ -65,10 +65,9 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
   } else {
     const int r = tid / XC, c = tid % XC;
     const int x0 = 4 * c;
-    constexpr int KP = (XR + 2) & 3, IEND = (XR + 3) & 3;
     const bool first = x0 == 0;
-    const bool kend = x0 == g.nx - 2 - KP;
-    const bool iend = x0 == g.nx - 1 - IEND;
+    constexpr int KP = (XR + 2) & 3, IEND = (XR + 3) & 3;
+    const bool kend = x0 == g.nx - 2 - KP, iend = x0 == g.nx - 1 - IEND;
     const int valid = iend ? IEND + 1 : 4;
     const exact::AxisSteps st{exact::axis_step(g.dx, g.rdx, g.rdx2),
                               exact::axis_step(g.dphi, g.rdphi, g.rdphi2),
@@ -86,27 +85,15 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
       const int rw0 = (32 * warp) / XC;
       const int rw1 = min((32 * warp + 31) / XC, it.r_eff - 1);
       exact::ItemCoef q;
-      q.iy = it.y0 + r;
-      q.nx = g.nx;
-      q.iv = it.iv;
-      q.nvp = g.nvp;
-      q.ie = it.ie;
-      q.nve = g.nve;
-      q.y_general = it.y0 + rw0 < 2 || it.y0 + rw1 + 2 >= g.nx;
-      q.v_general = it.iv < 2 || it.iv + 2 >= g.nvp;
-      q.e_general = it.ie < 2 || it.ie + 2 >= g.nve;
-      q.y = -g.extent + q.iy * g.dx;
-      q.vp = g.vp_lo + it.iv * g.dvp;
-      q.ve = g.ve_lo + it.ie * g.dve;
-      q.wp = fabs(q.vp) * g.curv_p;
-      q.we = fabs(q.ve) * g.curv_e;
-      q.acc_p = g.acc_p;
-      q.acc_e = g.acc_e;
-      q.dt = a.s.dt;
+      q.set(g, it.iv, it.ie, a.s.dt);
+      exact::RowCoef row;
+      row.iy = it.y0 + r;
+      row.y = -g.extent + row.iy * g.dx;
+      row.general = it.y0 + rw0 < 2 || it.y0 + rw1 + 2 >= g.nx;
       const unsigned base = og;  // issue index of own plane d = -2
       og += it.steps + 4;
       int64_t j = (((int64_t)(it.iv - g.slab_lo) * g.nve + it.ie) * g.nh + it.p0) * PP +
-                  (int64_t)q.iy * XP + x0;
+                  (int64_t)row.iy * XP + x0;
       auto own_at = [&](unsigned p) -> const float * {
         return own + (p & (OWN_SLOTS - 1)) * L.own_floats + ctr;
       };
@@ -131,11 +118,11 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
           exact::walk_hamiltonian<ORDER, XR>(
               *reinterpret_cast<const float2 *>(o0 - 2), C,
               *reinterpret_cast<const float2 *>(o0 + 4), own4(base + k + 3),
-              own4(base + k + 4), o0, XP, nb, L.nb_floats, first, kend, iend, xtab + x0,
-              cssn.x, cssn.y, q, st, carry, H);
+              own4(base + k + 4), o0, XP, nb, L.nb_floats, first, kend, iend, 0, 0,
+              xtab + x0, cssn.x, cssn.y, q, row, st, carry, H);
           const float4 P =
               BLEND ? *reinterpret_cast<const float4 *>(nb + NEIGHBOURS * L.nb_floats) : C;
-          bad |= exact::walk_update<ORDER, BLEND>(g, a.s, x0, it.p0 + k, j, valid, q,
+          bad |= exact::walk_update<ORDER, BLEND>(g, a.s, x0, it.p0 + k, j, valid, q, row,
                                                   xtab + x0, C, P, H, change);
         }
         mbar_arrive(&empty[slot]);  // release this step's set

@@ -78,3 +78,29 @@ def test_values_that_are_not_finite_are_reported(value):
         s.step(s.cfl_dt_limit)
         with pytest.raises(FloatingPointError):
             s.synchronize()
+
+
+@pytest.mark.parametrize("positions,headings,rows", [(17, 13, None), (18, 12, 18), (23, 7, 4),
+                                                     (33, 25, None), (40, 9, 11), (5, 4, None)])
+def test_tiled_batch_of_one_equals_the_single_grid(positions, headings, rows):
+    """Few items, so short heading chunks; every row remainder; tiles that do
+    not divide the rows or exceed what a CTA holds; two solves of unlike
+    length share the launch."""
+    from pursuit_evasion_b200.batch import BatchSolve, BatchSolver
+
+    grid = RelativeGrid(positions, headings, 5, 4, 3.0)
+    solves = [BatchSolve(A3, grid, 0.1), BatchSolve(A3, RelativeGrid(9, 8, 3, 3, 2.0), 0.03)]
+    with BatchSolver(solves) as b:
+        if rows:
+            b.set_tile(0, rows)
+        b.initialize()
+        b.run()
+        b.synchronize()
+        got = [(b.field(i), b.arrival(i), b.stats(i)) for i in range(2)]
+    for solve, (field, arrival, stats) in zip(solves, got):
+        with RelativeSolver(solve.config, solve.grid, local_precision="float64") as s:
+            s.initialize()
+            s.advance(solve.horizon)
+            np.testing.assert_array_equal(field.view(np.uint32), s.field().view(np.uint32))
+            np.testing.assert_array_equal(arrival.view(np.uint32), s.arrival().view(np.uint32))
+            assert stats == s.stats()
