@@ -23,6 +23,8 @@ struct pe_world {
   double t = 0;
   int64_t steps = 0;
   bool initialized = false;
+  bool column = false;  // the exact column kernel runs the stages
+  int tiny_turn = 0;    // which of stats->tiny_a0, tiny_a1 is the field's
   pe::LaunchTimer timer;  // launch times (profile / kernel_time)
 };
 
@@ -126,8 +128,26 @@ int read_stats(pe_world *h) {
   return PE_OK;
 }
 
-int stage(pe_world *h, const float *src, float *dst, const float *base, float dt) {
+unsigned *tiny_a(pe_world *h, int turn) {
+  return turn ? &h->stats->tiny_a1 : &h->stats->tiny_a0;
+}
+
+// The field in `a` was written from outside a stage: note whether it holds
+// values too small for the exact column kernel's quotients.
+int field_written(pe_world *h) {
+  h->tiny_turn = 0;
+  if (h->column) {
+    PE_CUDA_TRY(pe::world8_scan_tiny(h->g, h->a, tiny_a(h, 0), h->stream));
+    pe::count_launches(1);
+  }
+  return PE_OK;
+}
+
+int stage(pe_world *h, const float *src, float *dst, const float *base, float dt,
+          const unsigned *src_tiny, unsigned *dst_tiny) {
   pe::World8Stage s{};
+  s.src_tiny = src_tiny;
+  s.dst_tiny = dst_tiny;
   s.src = src;
   s.dst = dst;
   s.base = base;
@@ -144,27 +164,32 @@ int stage(pe_world *h, const float *src, float *dst, const float *base, float dt
   if (h->g.avoid_mode == 2 && !h->p_clear)
     return fail(PE_ESTATE, "avoid mode 2 needs pe_world_set_clearance first");
   cudaEvent_t e0 = h->timer.begin(h->stream);
-  PE_CUDA_TRY(h->p.fast ? pe::world8_stage_fast(h->g, s, h->stream)
-                        : pe::world8_stage(h->g, s, h->stream));
+  PE_CUDA_TRY(h->p.fast   ? pe::world8_stage_fast(h->g, s, h->stream)
+              : h->column ? pe::world8_stage_column(h->g, s, h->stream)
+                          : pe::world8_stage(h->g, s, h->stream));
   pe::count_launches(1);
   return h->timer.end(h->stream, e0, 0);
 }
 
 int step_impl(pe_world *h, double dt) {
-  PE_CUDA_TRY(cudaMemsetAsync(&h->stats->residual, 0, sizeof(unsigned long long),
-                              h->stream));
+  // one clear: the residual and every tiny word but the current field's
+  static_assert(sizeof(pe::World8Stats) == 24, "layout of World8Stats");
+  void *words = h->tiny_turn ? (void *)&h->stats->tiny_a0 : (void *)&h->stats->tiny_b;
+  PE_CUDA_TRY(cudaMemsetAsync(words, 0, 16, h->stream));
   const float dtf = (float)dt;  // native_world.cpp passes Real(dt)
+  unsigned *now = tiny_a(h, h->tiny_turn), *next = tiny_a(h, h->tiny_turn ^ 1);
   int rc;
   if (h->g.order == 1) {
-    rc = stage(h, h->a, h->b, nullptr, dtf);
+    rc = stage(h, h->a, h->b, nullptr, dtf, now, next);
     if (rc) return rc;
     std::swap(h->a, h->b);
   } else {
-    rc = stage(h, h->a, h->b, nullptr, dtf);
+    rc = stage(h, h->a, h->b, nullptr, dtf, now, &h->stats->tiny_b);
     if (rc) return rc;
-    rc = stage(h, h->b, h->a, h->a, dtf);
+    rc = stage(h, h->b, h->a, h->a, dtf, &h->stats->tiny_b, next);
     if (rc) return rc;
   }
+  h->tiny_turn ^= 1;
   h->t += dt;
   h->steps++;
   return PE_OK;
@@ -200,6 +225,7 @@ int pe_world_create(const pe_world_params *params, pe_world **out) {
   h->p = *params;
   h->g = make_grid(params);
   h->dt_limit = dt_limit(params, h->g);
+  h->column = !params->fast && pe::world8_column_exact_applies(h->g);
   const pe::World8Grid &g = h->g;
   // Axes exactly as native_world.cpp:138-150 (float), plus double trig.
   const double pi = std::acos(-1.0);
@@ -272,6 +298,8 @@ int pe_world_init_contact(pe_world *h, double p_length, double p_width,
                                       p_length, p_width, e_length, e_width, h->a,
                                       h->arrival, h->stream));
   pe::count_launches(1);
+  rc = field_written(h);
+  if (rc) return rc;
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->t = 0;
   h->steps = 0;
@@ -305,6 +333,8 @@ int pe_world_init_map(pe_world *h) {
   PE_CUDA_TRY(pe::world8_init_map(h->g, (float)h->p.capture_radius, h->p_clear, h->e_clear,
                                   h->a, h->arrival, h->stream));
   pe::count_launches(1);
+  rc = field_written(h);
+  if (rc) return rc;
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->t = 0;
   h->steps = 0;
@@ -319,6 +349,8 @@ int pe_world_init_square(pe_world *h) {
   PE_CUDA_TRY(pe::world8_init_square(h->g, h->x, (float)h->p.capture_radius, h->a,
                                      h->arrival, h->stream));
   pe::count_launches(1);
+  rc = field_written(h);
+  if (rc) return rc;
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->t = 0;
   h->steps = 0;
@@ -344,6 +376,8 @@ int pe_world_init_field(pe_world *h, const float *field, const float *arrival,
                                         h->stream));
     pe::count_launches(1);
   }
+  rc = field_written(h);
+  if (rc) return rc;
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->t = start_time;
   h->steps = 0;

@@ -54,7 +54,12 @@ __device__ __forceinline__ double quot2(double p, double v, double m, const Axis
 }
 // half a spacing times the smaller second difference, ties to the second
 __device__ __forceinline__ double edge_term(double a, double b, const AxisStep &s) {
-  return s.half * (fabs(a) < fabs(b) ? a : b);
+  double r;  // written out so that no integer sign masking is generated
+  asm("{\n .reg .pred p;\n .reg .f64 ua, ub;\n abs.f64 ua, %1;\n abs.f64 ub, %2;\n"
+      " setp.lt.f64 p, ua, ub;\n selp.f64 %0, %1, %2, p;\n}"
+      : "=d"(r)
+      : "d"(a), "d"(b));
+  return s.half * r;
 }
 
 __device__ __forceinline__ float f4_get(const float4 &v, int i) {
@@ -374,9 +379,11 @@ __device__ __forceinline__ bool walk_update(const Rel5Grid &g, const Rel5Stage &
   }
   bool bad = false;
   if (redo) {  // every cell of the chunk, in the general form
+    double ca = change.abs_max, cu = change.up_max;  // (the members stay in registers)
     for (int i = 0; i < valid; i++)
-      bad |= slow_cell<ORDER, BLEND>(g, s, x0 + i, row.iy, ip, q.iv, q.ie, j + i,
-                                     &change.abs_max, &change.up_max);
+      bad |= slow_cell<ORDER, BLEND>(g, s, x0 + i, row.iy, ip, q.iv, q.ie, j + i, &ca, &cu);
+    change.abs_max = ca;
+    change.up_max = cu;
     return bad;
   }
 #pragma unroll

@@ -25,10 +25,13 @@ struct World8Grid {
   float extent, arena, ap, ae, kp, ke;
 };
 
+// tiny_*: the field in a (two words, taken in turn) or b holds a nonzero value
+// below 2^-70; only the exact column kernel reads and sets them.  The order of
+// the words lets one 16-byte clear at a step's start leave the current field's.
 struct World8Stats {
+  unsigned int tiny_a0, tiny_b;
   unsigned long long residual;  // bits of a non-negative double
-  unsigned int nonfinite;
-  unsigned int pad;
+  unsigned int tiny_a1, nonfinite;
 };
 
 struct World8Stage {
@@ -41,6 +44,8 @@ struct World8Stage {
   double tau;
   World8Stats *stats;
   const float *p_clear;  // avoid_mode 2: pursuer clearance [xP][yP][thP]
+  const unsigned *src_tiny;  // exact column kernel: the words of src and dst
+  unsigned *dst_tiny;
 };
 
 // One stage in float32 arithmetic evaluated in the reference's order; the
@@ -48,6 +53,15 @@ struct World8Stage {
 // equal native_world.cpp's bit for bit.
 cudaError_t world8_stage(const World8Grid &g, const World8Stage &s,
                          cudaStream_t stream);
+
+// The same stage and bits by pursuer poses, the evader block in shared memory
+// (world8d_column_exact.cu); world8_column_exact_applies says for which grids,
+// world8_scan_tiny sets *tiny for a field that was just written.
+bool world8_column_exact_applies(const World8Grid &g);
+cudaError_t world8_stage_column(const World8Grid &g, const World8Stage &s,
+                                cudaStream_t stream);
+cudaError_t world8_scan_tiny(const World8Grid &g, const float *field, unsigned *tiny,
+                             cudaStream_t stream);
 
 // The same stage with reciprocal spacings and multiply-add contraction:
 // equal to the exact stage up to float rounding (and the ENO2 selections

@@ -79,6 +79,89 @@ __device__ __forceinline__ void slopes(const float *__restrict__ v, int64_t j,
   }
 }
 
+// Whether a stored value is nonzero and below 2^-70: differences of a field
+// without such values are zero or at least 2^-93, far from underflow in the
+// quotients by the spacings (world8d_column_exact.cu).
+__device__ __forceinline__ bool tiny_value(float v) {
+  return (__float_as_uint(v) & 0x7fffffffu) - 1u < 0x1C800000u - 1u;  // bits of 2^-70
+}
+
+// One cell of one stage: evader-block cell e_cell of pursuer pose o.
+template <bool FAST>
+__device__ __forceinline__ void stage_cell(const World8Grid &g, const World8Stage &s, int o,
+                                           int inner, int e_cell, float &change_max, bool &bad,
+                                           bool &tiny) {
+  const int64_t j = (int64_t)o * inner + e_cell;
+  int q[8];
+  {
+    int rest = o;
+    q[3] = rest % g.shape[3];
+    rest /= g.shape[3];
+    q[2] = rest % g.shape[2];
+    rest /= g.shape[2];
+    q[1] = rest % g.shape[1];
+    q[0] = rest / g.shape[1];
+    int e = e_cell;
+    q[7] = e % g.shape[7];
+    e /= g.shape[7];
+    q[6] = e % g.shape[6];
+    e /= g.shape[6];
+    q[5] = e % g.shape[5];
+    q[4] = e / g.shape[5];
+  }
+  const float vp = s.pv[q[3]];
+  const float palo = q[3] == 0 ? 0 : -g.ap;
+  const float pahi = q[3] == g.np - 1 ? 0 : g.ap;
+  const float fpx = vp * s.cs[q[2]], fpy = vp * s.sn[q[2]];
+  const float wp = fabsf(vp) * g.kp;
+  const float ve = s.ev[q[7]], we = fabsf(ve) * g.ke;
+  const float ealo = q[7] == 0 ? 0 : -g.ae;
+  const float eahi = q[7] == g.ne - 1 ? 0 : g.ae;
+  const float flow[8] = {fpx, fpy, 0, 0, ve * s.cs[q[6]], ve * s.sn[q[6]], 0, 0};
+  float grad[8], H = 0, diss = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    float lm, rp;
+    slopes<FAST>(s.src, j, g.stride[k], q[k], g.shape[k], g.spacing[k],
+                 g.inv_spacing[k], g.inv_spacing_sq[k], k == 2 || k == 6,
+                 g.linear_speed && (k == 3 || k == 7), g.order, lm, rp);
+    grad[k] = .5f * (lm + rp);
+    const float alpha = k == 2   ? wp
+                        : k == 3 ? g.ap
+                        : k == 6 ? we
+                        : k == 7 ? g.ae
+                                 : fabsf(flow[k]);
+    H += flow[k] * grad[k];
+    diss += .5f * alpha * (rp - lm);
+  }
+  const float p_lo_term = palo * grad[3], p_hi_term = pahi * grad[3];
+  const float e_lo_term = ealo * grad[7], e_hi_term = eahi * grad[7];
+  H += -wp * fabsf(grad[2]) + we * fabsf(grad[6]) +
+       (p_hi_term < p_lo_term ? p_hi_term : p_lo_term) +
+       (e_lo_term < e_hi_term ? e_hi_term : e_lo_term);
+  float value = s.src[j] + s.dt * (H + diss);
+  if (s.base) value = .5f * (s.base[j] + value);
+  if (g.order == 1 || s.base) {
+    const float previous = s.base ? s.base[j] : s.src[j];
+    // std::max(std::min(value, previous), avoid)
+    const float tube = previous < value ? previous : value;
+    float avoid = -INFINITY;
+    if (g.avoid_mode == 1) {
+      const float ax = fabsf(s.x[q[0]]), ay = fabsf(s.x[q[1]]);
+      avoid = (ax < ay ? ay : ax) - g.arena + 1e-6f;
+    } else if (g.avoid_mode == 2) {
+      avoid = -s.p_clear[(q[0] * g.n + q[1]) * g.nh + q[2]] + 1e-6f;
+    }
+    value = tube < avoid ? avoid : tube;
+    if (previous > 0 && value <= 0 && isnan(s.arrival[j]))
+      s.arrival[j] = (float)s.tau + s.dt * previous / (previous - value);
+    change_max = fmaxf(change_max, fabsf(value - previous));
+  }
+  if (!isfinite(value)) bad = true;
+  s.dst[j] = value;
+  tiny |= tiny_value(value);
+}
+
 template <bool FAST>
 // 6 CTAs of 256 threads per SM: the stage waits on its stencil loads, and
 // more warps hide them (7.45 against 7.74 ms per RK2 step at config 4)
@@ -92,74 +175,8 @@ __global__ void __launch_bounds__(256, 6)
   bool bad = false;
   for (int o = blockIdx.y; o < outer; o += gridDim.y) {
     if (e_cell < inner) {
-      const int64_t j = (int64_t)o * inner + e_cell;
-      int q[8];
-      {
-        int rest = o;
-        q[3] = rest % g.shape[3];
-        rest /= g.shape[3];
-        q[2] = rest % g.shape[2];
-        rest /= g.shape[2];
-        q[1] = rest % g.shape[1];
-        q[0] = rest / g.shape[1];
-        int e = e_cell;
-        q[7] = e % g.shape[7];
-        e /= g.shape[7];
-        q[6] = e % g.shape[6];
-        e /= g.shape[6];
-        q[5] = e % g.shape[5];
-        q[4] = e / g.shape[5];
-      }
-      const float vp = s.pv[q[3]];
-      const float palo = q[3] == 0 ? 0 : -g.ap;
-      const float pahi = q[3] == g.np - 1 ? 0 : g.ap;
-      const float fpx = vp * s.cs[q[2]], fpy = vp * s.sn[q[2]];
-      const float wp = fabsf(vp) * g.kp;
-      const float ve = s.ev[q[7]], we = fabsf(ve) * g.ke;
-      const float ealo = q[7] == 0 ? 0 : -g.ae;
-      const float eahi = q[7] == g.ne - 1 ? 0 : g.ae;
-      const float flow[8] = {fpx, fpy, 0, 0, ve * s.cs[q[6]], ve * s.sn[q[6]], 0, 0};
-      float grad[8], H = 0, diss = 0;
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        float lm, rp;
-        slopes<FAST>(s.src, j, g.stride[k], q[k], g.shape[k], g.spacing[k],
-                     g.inv_spacing[k], g.inv_spacing_sq[k], k == 2 || k == 6,
-                     g.linear_speed && (k == 3 || k == 7), g.order, lm, rp);
-        grad[k] = .5f * (lm + rp);
-        const float alpha = k == 2   ? wp
-                            : k == 3 ? g.ap
-                            : k == 6 ? we
-                            : k == 7 ? g.ae
-                                     : fabsf(flow[k]);
-        H += flow[k] * grad[k];
-        diss += .5f * alpha * (rp - lm);
-      }
-      const float p_lo_term = palo * grad[3], p_hi_term = pahi * grad[3];
-      const float e_lo_term = ealo * grad[7], e_hi_term = eahi * grad[7];
-      H += -wp * fabsf(grad[2]) + we * fabsf(grad[6]) +
-           (p_hi_term < p_lo_term ? p_hi_term : p_lo_term) +
-           (e_lo_term < e_hi_term ? e_hi_term : e_lo_term);
-      float value = s.src[j] + s.dt * (H + diss);
-      if (s.base) value = .5f * (s.base[j] + value);
-      if (g.order == 1 || s.base) {
-        const float previous = s.base ? s.base[j] : s.src[j];
-        // std::max(std::min(value, previous), avoid)
-        const float tube = previous < value ? previous : value;
-        float avoid = -INFINITY;
-        if (g.avoid_mode == 1) {
-          const float ax = fabsf(s.x[q[0]]), ay = fabsf(s.x[q[1]]);
-          avoid = (ax < ay ? ay : ax) - g.arena + 1e-6f;
-        } else if (g.avoid_mode == 2) {
-          avoid = -s.p_clear[(q[0] * g.n + q[1]) * g.nh + q[2]] + 1e-6f;
-        }
-        value = tube < avoid ? avoid : tube;
-        if (previous > 0 && value <= 0 && isnan(s.arrival[j]))
-          s.arrival[j] = (float)s.tau + s.dt * previous / (previous - value);
-        change_max = fmaxf(change_max, fabsf(value - previous));
-      }
-      if (!isfinite(value)) bad = true;
-      s.dst[j] = value;
+      bool tiny = false;
+      stage_cell<FAST>(g, s, o, inner, e_cell, change_max, bad, tiny);
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&s.stats->nonfinite, 1u);
