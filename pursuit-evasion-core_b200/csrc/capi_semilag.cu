@@ -25,7 +25,7 @@ struct pe_semilag {
   pe::SLStats *stats = nullptr, *host_stats = nullptr;
   // tiled value-only kernel (semilag5d_tiled.cu), when the grid allows it
   pe::SLSpeedStep *pstep = nullptr, *estep = nullptr;
-  uint8_t *hint = nullptr;
+  uint8_t *hint = nullptr;  // per cell: the last value backup's optimal pair
   pe::SLTiledPlan plan{};
   // per-item change flags of the last two tiled backups (work skipping)
   unsigned *changed[2] = {nullptr, nullptr};
@@ -186,9 +186,9 @@ bool use_tiled(const pe_semilag *h) {
   return h->kernel == PE_SL_KERNEL_AUTO && h->tiled_auto;
 }
 
-// Reset the per-cell action hints of the tiled kernel (neutral pair).
+// Reset the per-cell action hints (neutral pair).
 int reset_hints(pe_semilag *h) {
-  if (h->hint) PE_CUDA_TRY(cudaMemsetAsync(h->hint, 0x44, (size_t)h->g.n, h->stream));
+  PE_CUDA_TRY(cudaMemsetAsync(h->hint, 0x44, (size_t)h->g.n, h->stream));
   return PE_OK;
 }
 
@@ -204,10 +204,11 @@ int backup(pe_semilag *h, bool policy) {
   bk.earc = h->earc;
   bk.emove = h->emove;
   bk.stats = h->stats;
+  bk.hint = h->hint;
   cudaEvent_t e0 = h->timer.begin(h->stream);
   if (!policy && use_tiled(h)) {
     const bool skip = h->skip_enabled && h->skip_valid;
-    const pe::SLTiled tl{h->pstep, h->estep, h->hint,
+    const pe::SLTiled tl{h->pstep, h->estep,
                          skip ? h->changed[h->changed_cur] : nullptr,
                          h->changed[h->changed_cur ^ 1]};
     PE_CUDA_TRY(pe::sl_backup_tiled(h->g, bk, tl, h->plan, h->stream));
@@ -323,8 +324,10 @@ int pe_semilag_create(const pe_semilag_params *params, pe_semilag **out) {
                   tiled_geometry_ok(g, parc, earc, emove) &&
                   pe::sl_tiled_plan(g, optin - 1024, 0, &h->plan);
     // one CTA per SM: with fewer than ~8 items per SM the tail of the last
-    // wave and the per-item ring warm-up outweigh the gain (measured on a
-    // 33x24x11x11 grid: 1.46 ms tiled vs 0.81 ms generic per backup)
+    // wave and the per-item ring warm-up outweigh the gain, and the two kernels
+    // are about even where it ends (steady-state backups, generic / tiled:
+    // 33x24x11x11 0.57 / 1.00 ms, 49x36x15x15 3.12 / 3.15, 60x20x21x21 4.9 / 3.5,
+    // 65x48x21x21 13.7 / 8.9)
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, params->device);
     h->tiled_auto = h->tiled_ok && h->plan.items >= 8 * (int64_t)sms;
@@ -341,6 +344,7 @@ int pe_semilag_create(const pe_semilag_params *params, pe_semilag **out) {
   take(cudaMalloc(&h->plane, sizeof(float) * (size_t)g.sp));
   take(cudaMalloc(&h->pol_p, (size_t)g.n));
   take(cudaMalloc(&h->pol_e, (size_t)g.n));
+  take(cudaMalloc(&h->hint, (size_t)g.n));
   take(cudaMalloc(&h->parc, sizeof(pe::SLPursuerArc) * parc.size()));
   take(cudaMalloc(&h->earc, sizeof(pe::SLEvaderArc) * earc.size()));
   take(cudaMalloc(&h->emove, sizeof(pe::SLEvaderMove) * emove.size()));
@@ -358,7 +362,6 @@ int pe_semilag_create(const pe_semilag_params *params, pe_semilag **out) {
   if (err == cudaSuccess && h->tiled_ok) {
     take(cudaMalloc(&h->pstep, sizeof(pe::SLSpeedStep) * pstep.size()));
     take(cudaMalloc(&h->estep, sizeof(pe::SLSpeedStep) * estep.size()));
-    take(cudaMalloc(&h->hint, (size_t)g.n));
     // flags for the finest possible tiling (one row per tile)
     const size_t flags = sizeof(unsigned) * (size_t)g.nvp * g.nve * g.nx;
     take(cudaMalloc(&h->changed[0], flags));

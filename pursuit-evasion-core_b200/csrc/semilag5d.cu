@@ -37,90 +37,116 @@ __device__ __forceinline__ void locate_clamped(float f, int n, int &j, float &w)
   w = f - (float)k;
 }
 
+// One (pursuer action, evader reply) pair of a block's (vP, vE, psi): what the
+// successor and its interpolation need beyond the cell's position.
+struct GenericPair {
+  float px, py, c, s, ex, ey;  // displacements and the pursuer's turn
+  float wv, we, wp;            // upper weights of vP, vE and psi
+  int64_t base;                // lower corner's offset at (y, x) = (0, 0)
+  int64_t dpsi;                // from the lower to the upper heading
+};
+
+// Value interpolated at the successor of the cell at (x, y).
+__device__ __forceinline__ float pair_successor(const SLGrid &g, const float *__restrict__ V,
+                                                const GenericPair &p, float x, float y) {
+  const float dxp = x + p.ex - p.px, dyp = y + p.ey - p.py;
+  const float xr = fmaf(p.c, dxp, p.s * dyp);
+  const float yr = fmaf(p.c, dyp, -p.s * dxp);
+  int jx, jy;
+  float wx, wy;
+  locate_clamped((xr + g.extent) * g.ihx, g.nx, jx, wx);
+  locate_clamped((yr + g.extent) * g.ihx, g.nx, jy, wy);
+  const float *at = V + p.base + (int64_t)jy * g.sy + jx;
+  float value = 0.f;
+#pragma unroll
+  for (int bv = 0; bv < 2; bv++) {
+    const float w_v = bv ? p.wv : 1.f - p.wv;
+    if (w_v == 0.f) continue;
+#pragma unroll
+    for (int be = 0; be < 2; be++) {
+      const float w_e = be ? p.we : 1.f - p.we;
+      if (w_e == 0.f) continue;
+      float acc_p = 0.f;
+#pragma unroll
+      for (int bp = 0; bp < 2; bp++) {
+        const float *q = at + bv * g.sv + be * g.se + (bp ? p.dpsi : 0);
+        const float v00 = __ldg(q), v01 = __ldg(q + 1);
+        const float v10 = __ldg(q + g.sy), v11 = __ldg(q + g.sy + 1);
+        const float r0 = fmaf(wx, v01 - v00, v00);
+        const float r1 = fmaf(wx, v11 - v10, v10);
+        const float plane = fmaf(wy, r1 - r0, r0);
+        acc_p = bp ? fmaf(p.wp, plane - acc_p, acc_p) : plane;
+      }
+      value = fmaf(w_v * w_e, acc_p, value);
+    }
+  }
+  if (g.mode == SL_MINTIME) value = fminf(fmaxf(value, 0.f), 1.f);
+  return value;
+}
+
+// Value-only backups take the pairs in an order guided by the previous
+// backup's optimal pair (hint: its pursuer action first, its evader reply
+// first against every action): the minimum and the maxima do not depend on
+// the order, but an action that cannot win is then abandoned after its first
+// reply.  Each lane walks its own sequence, so a warp runs as long as its
+// longest lane and not as the sum over actions of the longest.  33x24x11x11
+// tube backups in steady state: 1600 -> 566 us (catalogue order, arcs decoded per
+// evaluation, before).
 template <bool POLICY>
 __global__ void __launch_bounds__(128)
     sl_backup_kernel(const SLGrid g, const SLBackup b) {
-  __shared__ SLPursuerArc sp[9];
-  __shared__ SLEvaderArc se[9];
-  __shared__ SLEvaderMove sm[9];
+  __shared__ GenericPair pairs[81];
   __shared__ float warp_max[4];
   const int ip = blockIdx.y;
   const int ie = blockIdx.z % g.nve, iv = blockIdx.z / g.nve;
-  if (threadIdx.x < 9) {
-    sp[threadIdx.x] = b.parc[iv * 9 + threadIdx.x];
-    se[threadIdx.x] = b.earc[ie * 9 + threadIdx.x];
-    sm[threadIdx.x] = b.emove[((int64_t)ip * g.nve + ie) * 9 + threadIdx.x];
+  if (threadIdx.x < 81) {
+    const int up = threadIdx.x / 9, ue = threadIdx.x % 9;
+    const SLPursuerArc pa = b.parc[iv * 9 + up];
+    const SLEvaderArc ea = b.earc[ie * 9 + ue];
+    const SLEvaderMove em = b.emove[((int64_t)ip * g.nve + ie) * 9 + ue];
+    GenericPair p;
+    p.px = pa.px;
+    p.py = pa.py;
+    p.c = pa.c;
+    p.s = pa.s;
+    p.ex = em.ex;
+    p.ey = em.ey;
+    int jv, je;
+    locate_clamped(pa.fv, g.nvp, jv, p.wv);
+    locate_clamped(ea.fv, g.nve, je, p.we);
+    const float fpsi = (float)ip + (ea.turn_idx - pa.turn_idx);
+    const float fl = floorf(fpsi);
+    p.wp = fpsi - fl;
+    int jp = (int)fl % g.nh;
+    jp += jp < 0 ? g.nh : 0;
+    const int jp1 = jp + 1 == g.nh ? 0 : jp + 1;
+    p.base = (int64_t)jv * g.sv + (int64_t)je * g.se + (int64_t)jp * g.sp;
+    p.dpsi = (int64_t)(jp1 - jp) * g.sp;
+    pairs[threadIdx.x] = p;
   }
   __syncthreads();
   const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = cell < g.nx * g.nx;
   float change = 0.f;
   bool bad = false;
-  if (cell < g.nx * g.nx) {
-    const int ix = cell % g.nx, iy = cell / g.nx;
-    const float x = fmaf((float)ix, g.dx, -g.extent);
-    const float y = fmaf((float)iy, g.dx, -g.extent);
-    const int64_t j = (int64_t)blockIdx.z * g.se + (int64_t)ip * g.sp + cell;
-    const float *__restrict__ V = b.src;
-    const float current = V[j];
-    float best = (g.mode == SL_TUBE) ? current : INFINITY;
-    float worst_of[9];
-    int e_of[9];
-    for (int up = 0; up < 9; up++) {
-      const SLPursuerArc pa = sp[up];
-      // pursuer speed corner(s)
-      int jv;
-      float wv;
-      locate_clamped(pa.fv, g.nvp, jv, wv);
-      float worst = -INFINITY;
-      float vals[POLICY ? 9 : 1];
-      for (int ue = 0; ue < 9; ue++) {
-        const SLEvaderArc ea = se[ue];
-        const SLEvaderMove em = sm[ue];
-        const float dxp = x + em.ex - pa.px, dyp = y + em.ey - pa.py;
-        const float xr = fmaf(pa.c, dxp, pa.s * dyp);
-        const float yr = fmaf(pa.c, dyp, -pa.s * dxp);
-        int jx, jy, je;
-        float wx, wy, we;
-        locate_clamped((xr + g.extent) * g.ihx, g.nx, jx, wx);
-        locate_clamped((yr + g.extent) * g.ihx, g.nx, jy, wy);
-        locate_clamped(ea.fv, g.nve, je, we);
-        const float fpsi = (float)ip + (ea.turn_idx - pa.turn_idx);
-        const float fl = floorf(fpsi);
-        const float wp = fpsi - fl;
-        int jp = (int)fl % g.nh;
-        jp += jp < 0 ? g.nh : 0;
-        const int jp1 = jp + 1 == g.nh ? 0 : jp + 1;
-        float value = 0.f;
-#pragma unroll
-        for (int bv = 0; bv < 2; bv++) {
-          const float w_v = bv ? wv : 1.f - wv;
-          if (w_v == 0.f) continue;
-#pragma unroll
-          for (int be = 0; be < 2; be++) {
-            const float w_e = be ? we : 1.f - we;
-            if (w_e == 0.f) continue;
-            const int64_t speed_base = (int64_t)(jv + bv) * g.sv + (int64_t)(je + be) * g.se;
-            float acc_p = 0.f;
-#pragma unroll
-            for (int bp = 0; bp < 2; bp++) {
-              const int64_t pb = speed_base + (int64_t)(bp ? jp1 : jp) * g.sp +
-                                 (int64_t)jy * g.sy + jx;
-              const float v00 = __ldg(V + pb), v01 = __ldg(V + pb + 1);
-              const float v10 = __ldg(V + pb + g.sy), v11 = __ldg(V + pb + g.sy + 1);
-              const float r0 = fmaf(wx, v01 - v00, v00);
-              const float r1 = fmaf(wx, v11 - v10, v10);
-              const float plane = fmaf(wy, r1 - r0, r0);
-              acc_p = bp ? fmaf(wp, plane - acc_p, acc_p) : plane;
-            }
-            value = fmaf(w_v * w_e, acc_p, value);
-          }
+  const int ix = cell % g.nx, iy = cell / g.nx;
+  const float x = fmaf((float)ix, g.dx, -g.extent);
+  const float y = fmaf((float)iy, g.dx, -g.extent);
+  const int64_t j = (int64_t)blockIdx.z * g.se + (int64_t)ip * g.sp + cell;
+  const float *__restrict__ V = b.src;
+  const float current = live ? V[j] : 0.f;
+  float best = (g.mode == SL_TUBE) ? current : INFINITY;
+  if (POLICY) {
+    if (live) {
+      float worst_of[9];
+      int e_of[9];
+      for (int up = 0; up < 9; up++) {
+        float worst = -INFINITY;
+        float vals[9];
+        for (int ue = 0; ue < 9; ue++) {
+          vals[ue] = pair_successor(g, V, pairs[up * 9 + ue], x, y);
+          worst = fmaxf(worst, vals[ue]);
         }
-        if (g.mode == SL_MINTIME) value = fminf(fmaxf(value, 0.f), 1.f);
-        if (POLICY) vals[ue] = value;
-        worst = fmaxf(worst, value);
-        if (!POLICY && worst >= best) break;  // cannot lower the minimum
-      }
-      if (POLICY) {
         worst_of[up] = worst;
         int pick = kEvaderOrder[0];
 #pragma unroll
@@ -130,17 +156,8 @@ __global__ void __launch_bounds__(128)
             break;
           }
         e_of[up] = pick;
+        best = fminf(best, worst);
       }
-      best = fminf(best, worst);
-    }
-    float out;
-    if (g.mode == SL_TUBE) {
-      out = best;
-    } else {
-      const float d = hypotf(x, y) - g.radius;  // capture test of this cell
-      out = d <= 0.f ? 0.f : fmaf(g.beta, best, 1.f - g.beta);
-    }
-    if (POLICY) {
       float lo = INFINITY;
       for (int up = 0; up < 9; up++) lo = fminf(lo, worst_of[up]);
       int pick = 0, key = 1 << 30;
@@ -154,6 +171,43 @@ __global__ void __launch_bounds__(128)
       }
       b.policy_p[j] = (uint8_t)pick;
       b.policy_e[j] = (uint8_t)e_of[pick];
+    }
+  } else {
+    const int h = live ? (int)b.hint[j] : 0x44;
+    const int hu = (h >> 4) < 9 ? h >> 4 : 4, he = (h & 15) < 9 ? h & 15 : 4;
+    int i = live ? 0 : 9, r = 0;  // places in the sequences of actions and replies
+    int bu = hu, be = he, arg = he;
+    float worst = -INFINITY;
+    while (__any_sync(0xffffffffu, i < 9)) {
+      if (i < 9) {
+        const int up = i == 0 ? hu : i - (i <= hu), ue = r == 0 ? he : r - (r <= he);
+        const float value = pair_successor(g, V, pairs[up * 9 + ue], x, y);
+        if (value > worst) arg = ue;
+        worst = fmaxf(worst, value);
+        if (worst >= best || ++r == 9) {  // cannot lower the minimum, or complete
+          if (worst < best) {
+            best = worst;
+            bu = up;
+            be = arg;
+          } else if (i == 0) {
+            be = arg;  // the reply that settled the hinted action
+          }
+          best = fminf(best, worst);
+          worst = -INFINITY;
+          r = 0;
+          i++;
+        }
+      }
+    }
+    if (live) b.hint[j] = (uint8_t)((bu << 4) | be);
+  }
+  if (live) {
+    float out;
+    if (g.mode == SL_TUBE) {
+      out = best;
+    } else {
+      const float d = hypotf(x, y) - g.radius;  // capture test of this cell
+      out = d <= 0.f ? 0.f : fmaf(g.beta, best, 1.f - g.beta);
     }
     if (!isfinite(out)) bad = true;
     b.dst[j] = out;

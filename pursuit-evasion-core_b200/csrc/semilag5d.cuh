@@ -52,6 +52,8 @@ struct SLBackup {
   const SLEvaderArc *earc;
   const SLEvaderMove *emove;
   SLStats *stats;
+  uint8_t *hint;  // [cells]: (pursuer action << 4) | evader reply of the previous
+                  // value backup; 0x44 before the first
 };
 
 cudaError_t sl_backup(const SLGrid &g, const SLBackup &b, cudaStream_t stream);
@@ -72,8 +74,6 @@ struct SLSpeedStep {
 struct SLTiled {
   const SLSpeedStep *pstep;  // [nvp]
   const SLSpeedStep *estep;  // [nve]
-  uint8_t *hint;             // [cells]: (pursuer action << 4) | evader reply of
-                             // the previous backup; 0x44 before the first
   // Work skipping: changed_in[item] != 0 where some cell of the item changed
   // (in its bits) in the previous backup; an item whose 3x3x3 neighbourhood
   // of items (vP, vE, y tile +-1) did not change reads the same inputs as

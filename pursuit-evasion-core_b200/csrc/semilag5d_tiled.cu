@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(SL_TILED_MAX_THREADS, 1)
         const int iy = ty0 + row;
         const int64_t cell = plane_base + (int64_t)row * nx + col;
         const float cur = valid ? b.src[cell] : 0.f;
-        const int h = valid ? (int)t.hint[cell] : 0x44;
+        const int h = valid ? (int)b.hint[cell] : 0x44;
         const float x = fmaf((float)col, g.dx, -g.extent);
         const float y = fmaf((float)iy, g.dx, -g.extent);
         const bool captured = MODE == SL_MINTIME && hypotf(x, y) - g.radius <= 0.f;
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(SL_TILED_MAX_THREADS, 1)
           if (!isfinite(out)) bad = true;
           item_changed |= __float_as_uint(out) != __float_as_uint(cur);
           b.dst[cell] = out;
-          t.hint[cell] = (uint8_t)((bu << 4) | be);
+          b.hint[cell] = (uint8_t)((bu << 4) | be);
           change = fmaxf(change, fabsf(out - cur));
         }
       }
