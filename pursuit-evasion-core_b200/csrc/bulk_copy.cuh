@@ -4,6 +4,8 @@
 // persistent stage kernels that stream planes into shared-memory rings.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace pe {
@@ -86,6 +88,35 @@ __device__ __forceinline__ bool wait_phase(uint64_t *bar, uint32_t parity,
     if (mbar_try_wait(bar, parity)) return true;
   atomicOr(timeout_flag, 1u);
   return false;
+}
+
+// Programmatic dependent launch: lets the stream's next kernel start its
+// prologue while this one runs, and waits for the kernels before this one to
+// be complete (their stores visible).
+__device__ __forceinline__ void grid_launch_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launch `kernel`, with `overlap` so that its prologue may run under the
+// stream's previous kernel; the kernel calls grid_wait_previous before it
+// touches what that one writes.
+template <class... Params, class... Args>
+cudaError_t launch_overlapped(bool overlap, void (*kernel)(Params...), dim3 grid, int threads,
+                              size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace bulk

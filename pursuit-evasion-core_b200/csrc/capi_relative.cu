@@ -93,8 +93,6 @@ int launch_stage(pe_relative *h, int stage, const float *src, float *dst,
 }
 
 int step_impl(pe_relative *h, double dt) {
-  PE_CUDA_TRY(cudaMemsetAsync(&h->stats->residual, 0, sizeof(unsigned long long),
-                              h->stream));
   int rc;
   if (h->g.order == 1) {
     rc = launch_stage(h, 0, h->a, h->b, dt, 0);

@@ -225,9 +225,6 @@ int pe_relative_shard_stage(pe_relative_shard *h, int32_t stage, double dt) {
   if (!h->initialized) return fail(PE_ESTATE, "stage before init");
   if (stage < 0 || stage >= h->g.order) return fail(PE_EINVAL, "stage must be in [0, order)");
   if (!(dt > 0) || !std::isfinite(dt)) return fail(PE_EINVAL, "dt must be positive");
-  if (stage == 0)
-    PE_CUDA_TRY(cudaMemsetAsync(&h->stats->residual, 0, sizeof(unsigned long long),
-                                h->stream));
   pe::Rel5Stage s{};
   const int blend = stage == 1;
   s.src = blend ? h->b : h->a;

@@ -94,6 +94,8 @@ int rel5_last_resident_ctas();
 // Whether a tile fits the kernel's limits (threads, shared memory).
 bool rel5_tile_valid(const Rel5Grid &g, const Rel5Tile &t);
 
+// Every stage function clears the residual word at a step's first stage.
+//
 // Fast path: float32 local arithmetic.  blend = 0 for stage 1 (or the only
 // stage of RK1), 1 for the RK2 averaging stage.
 cudaError_t rel5_stage_f32(const Rel5Grid &g, const Rel5Tile &t,

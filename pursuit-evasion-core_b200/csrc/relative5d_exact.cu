@@ -11,6 +11,7 @@
 // it runs 12 CTAs of 128 threads per SM at 40 registers, spills included:
 // 3.70 / 4.30 ms per stage at config 2 against 5.51 / 6.54 ms at 6 CTAs per
 // SM (76-80 registers), same results.
+#include "bulk_copy.cuh"
 #include "relative5d_exact.cuh"
 
 namespace pe {
@@ -20,7 +21,11 @@ template <int ORDER, int BLEND, typename T = float>
 __global__ void __launch_bounds__(128, 12)
     rel5_stage_exact_kernel(const Rel5Grid g, const Rel5Stage s) {
   __shared__ double scratch[4];
+  bulk::grid_launch_next();
+  bulk::grid_wait_previous();  // the fields the stage before this one wrote
   const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+  // the step's residual starts at its second stage: clear it in the first
+  if (ORDER == 2 && !BLEND && (cell | blockIdx.y | blockIdx.z) == 0) s.stats->residual = 0ull;
   double change_abs = 0, change_up = 0;
   bool bad = false;
   if (cell < g.nx * g.nx) {
@@ -64,13 +69,15 @@ cudaError_t rel5_stage_f64_storage(const Rel5Grid &g, const Rel5Stage &s, int bl
                                    cudaStream_t stream) {
   const int threads = 128;
   const dim3 grid((g.nx * g.nx + threads - 1) / threads, g.nvp * g.nve, g.nh);
+  const bool overlap = g.se * g.nve * g.nvp < 1000000;
   if (g.order == 1)
-    rel5_stage_exact_kernel<1, 0, double><<<grid, threads, 0, stream>>>(g, s);
-  else if (blend)
-    rel5_stage_exact_kernel<2, 1, double><<<grid, threads, 0, stream>>>(g, s);
-  else
-    rel5_stage_exact_kernel<2, 0, double><<<grid, threads, 0, stream>>>(g, s);
-  return cudaGetLastError();
+    return bulk::launch_overlapped(overlap, rel5_stage_exact_kernel<1, 0, double>, grid, threads, 0,
+                                   stream, g, s);
+  if (blend)
+    return bulk::launch_overlapped(overlap, rel5_stage_exact_kernel<2, 1, double>, grid, threads, 0,
+                                   stream, g, s);
+  return bulk::launch_overlapped(overlap, rel5_stage_exact_kernel<2, 0, double>, grid, threads,
+                                 0, stream, g, s);
 }
 
 cudaError_t rel5_stage_f64(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s, int blend,
@@ -79,13 +86,19 @@ cudaError_t rel5_stage_f64(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage
   const int threads = 128;
   const int slabs = g.own_n > 0 ? g.own_n : g.nvp;
   const dim3 grid((g.nx * g.nx + threads - 1) / threads, slabs * g.nve, g.nh);
-  if (g.order == 1)
-    rel5_stage_exact_kernel<1, 0><<<grid, threads, 0, stream>>>(g, s);
-  else if (blend)
-    rel5_stage_exact_kernel<2, 1><<<grid, threads, 0, stream>>>(g, s);
-  else
-    rel5_stage_exact_kernel<2, 0><<<grid, threads, 0, stream>>>(g, s);
-  return cudaGetLastError();
+  const bool overlap = g.se * g.nve * slabs < 1000000;  // (short stages: ring_args)
+  if (g.order == 1) {  // (an RK2 step's first stage clears the residual itself)
+    const cudaError_t e =
+        cudaMemsetAsync(&s.stats->residual, 0, sizeof(unsigned long long), stream);
+    if (e != cudaSuccess) return e;
+    return bulk::launch_overlapped(overlap, rel5_stage_exact_kernel<1, 0>, grid, threads, 0,
+                                   stream, g, s);
+  }
+  if (blend)
+    return bulk::launch_overlapped(overlap, rel5_stage_exact_kernel<2, 1>, grid, threads, 0,
+                                   stream, g, s);
+  return bulk::launch_overlapped(overlap, rel5_stage_exact_kernel<2, 0>, grid, threads, 0,
+                                 stream, g, s);
 }
 
 }  // namespace pe

@@ -90,7 +90,7 @@ __device__ __forceinline__ void sum_jump4(float4 m2, float4 m1, float4 v, float4
 // start the item's heading differences at step 0.
 //
 // XR = nx mod 4 places the x end rules (see slopes_x_fixed).
-template <int ORDER, int BLEND, int XR, int XPC, int RC>
+template <int ORDER, int BLEND, int XR, int XPC, int RC, bool OVERLAP>
 __global__ void __launch_bounds__(TARGET_THREADS, 2)
     rel5_stage_kernel(const RingArgs a) {
   extern __shared__ __align__(128) float smem[];
@@ -126,6 +126,12 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
   for (int k = tid; k < g.nh; k += blockDim.x) {
     trig[2 * k] = __ldg(a.s.csf + k);
     trig[2 * k + 1] = __ldg(a.s.snf + k);
+  }
+  if (OVERLAP) {
+    grid_launch_next();
+    grid_wait_previous();  // the fields the stage before this one wrote
+    // the step's residual starts at its second stage: clear it in the first
+    if (ORDER == 2 && !BLEND && blockIdx.x == 0 && tid == 0) a.s.stats->residual = 0ull;
   }
   __syncthreads();
 
@@ -442,19 +448,19 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
 
 int g_last_resident = 0;
 
-template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0>
+template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0, bool OVERLAP = false>
 cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
   // Resident CTAs per SM for this (shared memory, block size); recomputed
   // when either changes.
   static int configured_smem = 0, configured_threads = 0;
   static int resident = 0;
   if (configured_smem != (int)smem || configured_threads != threads || resident == 0) {
-    cudaError_t e = cudaFuncSetAttribute(rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC>,
+    cudaError_t e = cudaFuncSetAttribute(rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &resident, rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC>, threads, smem);
+        &resident, rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>, threads, smem);
     if (e != cudaSuccess) return e;
     if (resident < 1) return cudaErrorInvalidConfiguration;
     configured_smem = (int)smem;
@@ -465,22 +471,28 @@ cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const int blocks = std::min(args.items, sms * resident);
   g_last_resident = resident;
-  rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC><<<blocks, threads, smem, stream>>>(args);
-  return cudaGetLastError();
+  return launch_overlapped(OVERLAP, rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>,
+                           dim3((unsigned)blocks), threads, smem, stream, args);
+}
+
+template <int ORDER, int BLEND, bool OVERLAP>
+cudaError_t launch_nx(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
+  switch (args.g.nx & 3) {
+    case 0: return launch_xr<ORDER, BLEND, 0, 0, 0, OVERLAP>(args, smem, threads, stream);
+    case 1: return launch_xr<ORDER, BLEND, 1, 0, 0, OVERLAP>(args, smem, threads, stream);
+    case 2: return launch_xr<ORDER, BLEND, 2, 0, 0, OVERLAP>(args, smem, threads, stream);
+    default: return launch_xr<ORDER, BLEND, 3, 0, 0, OVERLAP>(args, smem, threads, stream);
+  }
 }
 
 template <int ORDER, int BLEND>
 cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
   // the 65-position grids (68-float rows) at the default 13-row tile, with
   // compile-time offsets (5 % faster on the 89M-cell grid, B200)
-  if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13)
+  if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13 && !args.overlap)
     return launch_xr<ORDER, BLEND, 1, 68, 13>(args, smem, threads, stream);
-  switch (args.g.nx & 3) {
-    case 0: return launch_xr<ORDER, BLEND, 0>(args, smem, threads, stream);
-    case 1: return launch_xr<ORDER, BLEND, 1>(args, smem, threads, stream);
-    case 2: return launch_xr<ORDER, BLEND, 2>(args, smem, threads, stream);
-    default: return launch_xr<ORDER, BLEND, 3>(args, smem, threads, stream);
-  }
+  return args.overlap ? launch_nx<ORDER, BLEND, true>(args, smem, threads, stream)
+                      : launch_nx<ORDER, BLEND, false>(args, smem, threads, stream);
 }
 
 __global__ void rel5_init_kernel(const float *__restrict__ plane, int64_t plane_size,
@@ -613,6 +625,8 @@ cudaError_t rel5_stage_f32(const Rel5Grid &g, const Rel5Tile &t,
   const RingArgs args = ring_args(g, t, s);
   const int threads = 32 * (args.consumer_warps + 1);
   const size_t smem = rel5_fast_smem_bytes(g, t);
+  const cudaError_t e = ring::clear_residual(args, blend, stream);
+  if (e != cudaSuccess) return e;
   if (g.order == 1) return launch<1, 0>(args, smem, threads, stream);
   if (blend) return launch<2, 1>(args, smem, threads, stream);
   return launch<2, 0>(args, smem, threads, stream);

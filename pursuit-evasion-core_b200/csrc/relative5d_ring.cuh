@@ -43,6 +43,7 @@ struct RingArgs {
   int vp_first, vp_count;  // the vP slabs this launch updates (a shard's own)
   float ihx, ihp, ihv, ihe;
   float dt;
+  bool overlap;  // launch under the previous kernel's tail (short stages)
 };
 
 // Shared memory layout of one CTA.
@@ -180,7 +181,19 @@ inline RingArgs ring_args(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage 
   args.ihv = (float)(1.0 / g.dvp);
   args.ihe = (float)(1.0 / g.dve);
   args.dt = (float)s.dt;
+  // Short stages, where launch latency counts: the 16 RK2 steps of a 17x12x7x7
+  // solve take 415 us without and 342 us with it.  Long ones lose by it, since the
+  // next stage's CTAs then fill the SMs unevenly as this one's leave
+  // (33x24x11x11 exact 12.95 against 13.3 ms, 65x48x21x21 float32 71.7 against
+  // 73.2 ms per solve).
+  args.overlap = rel5_tile_cost(g, t) < 12;
   return args;
+}
+
+// Clear the step's residual before its first stage, unless the kernel does.
+inline cudaError_t clear_residual(const RingArgs &a, int blend, cudaStream_t stream) {
+  if (blend || (a.overlap && a.g.order == 2)) return cudaSuccess;
+  return cudaMemsetAsync(&a.s.stats->residual, 0, sizeof(unsigned long long), stream);
 }
 
 }  // namespace ring

@@ -24,7 +24,7 @@ using namespace ring;
 // heading (cos, sin) pairs and x positions, in double
 __host__ __device__ inline int table_bytes(const Rel5Grid &g) { return 16 * g.nh + 8 * g.xp; }
 
-template <int ORDER, int BLEND, int XR, int XPC, int RC>
+template <int ORDER, int BLEND, int XR, int XPC, int RC, bool OVERLAP>
 __global__ void __launch_bounds__(TARGET_THREADS, 2)
     rel5_walk_exact_kernel(const __grid_constant__ RingArgs a) {
   extern __shared__ __align__(128) float smem[];
@@ -55,6 +55,12 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
   for (int k = tid; k < g.nh; k += blockDim.x)
     trig[k] = make_double2(__ldg(a.s.cs + k), __ldg(a.s.sn + k));
   for (int k = tid; k < XP; k += blockDim.x) xtab[k] = -g.extent + k * g.dx;
+  if (OVERLAP) {
+    grid_launch_next();
+    grid_wait_previous();  // the fields the stage before this one wrote
+    // the step's residual starts at its second stage: clear it in the first
+    if (ORDER == 2 && !BLEND && blockIdx.x == 0 && tid == 0) a.s.stats->residual = 0ull;
+  }
   __syncthreads();
 
   bool bad = false;
@@ -147,9 +153,9 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
   }
 }
 
-template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0>
+template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0, bool OVERLAP = false>
 cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
-  auto kernel = rel5_walk_exact_kernel<ORDER, BLEND, XR, XPC, RC>;
+  auto kernel = rel5_walk_exact_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>;
   // co-resident CTAs of the last (device, shared memory, block size) this
   // thread launched
   struct Shape {
@@ -170,20 +176,27 @@ cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream
     if (resident < 1) return cudaErrorInvalidConfiguration;
     last = Shape{device, (int)smem, threads, sms * resident};
   }
-  kernel<<<std::min(args.items, last.ctas), threads, smem, stream>>>(args);
-  return cudaGetLastError();
+  return launch_overlapped(OVERLAP, kernel,
+                           dim3((unsigned)std::min(args.items, last.ctas)), threads, smem,
+                           stream, args);
+}
+
+template <int ORDER, int BLEND, bool OVERLAP>
+cudaError_t launch_nx(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
+  switch (args.g.nx & 3) {
+    case 0: return launch_xr<ORDER, BLEND, 0, 0, 0, OVERLAP>(args, smem, threads, stream);
+    case 1: return launch_xr<ORDER, BLEND, 1, 0, 0, OVERLAP>(args, smem, threads, stream);
+    case 2: return launch_xr<ORDER, BLEND, 2, 0, 0, OVERLAP>(args, smem, threads, stream);
+    default: return launch_xr<ORDER, BLEND, 3, 0, 0, OVERLAP>(args, smem, threads, stream);
+  }
 }
 
 template <int ORDER, int BLEND>
 cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
-  if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13)
+  if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13 && !args.overlap)
     return launch_xr<ORDER, BLEND, 1, 68, 13>(args, smem, threads, stream);
-  switch (args.g.nx & 3) {
-    case 0: return launch_xr<ORDER, BLEND, 0>(args, smem, threads, stream);
-    case 1: return launch_xr<ORDER, BLEND, 1>(args, smem, threads, stream);
-    case 2: return launch_xr<ORDER, BLEND, 2>(args, smem, threads, stream);
-    default: return launch_xr<ORDER, BLEND, 3>(args, smem, threads, stream);
-  }
+  return args.overlap ? launch_nx<ORDER, BLEND, true>(args, smem, threads, stream)
+                      : launch_nx<ORDER, BLEND, false>(args, smem, threads, stream);
 }
 
 }  // namespace
@@ -209,6 +222,8 @@ cudaError_t rel5_stage_f64_tiled(const Rel5Grid &g, const Rel5Tile &t, const Rel
   const RingArgs args = ring_args(g, t, s);
   const int threads = 32 * (args.consumer_warps + 1);
   const size_t smem = (size_t)smem_layout(t.rows, g.xp, table_bytes(g)).bytes;
+  const cudaError_t e = ring::clear_residual(args, blend, stream);
+  if (e != cudaSuccess) return e;
   if (g.order == 1) return launch<1, 0>(args, smem, threads, stream);
   if (blend) return launch<2, 1>(args, smem, threads, stream);
   return launch<2, 0>(args, smem, threads, stream);
