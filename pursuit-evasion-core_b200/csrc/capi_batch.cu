@@ -223,8 +223,7 @@ int copy_out(pe_batch *h, int32_t solve, float *host, bool arrival) {
   PE_CUDA_TRY(pe::rel5_pack(g, arrival ? field_arrival(h, solve) : field_a(h, solve), dense,
                             h->stream));
   pe::count_launches(1);
-  PE_CUDA_TRY(cudaMemcpyAsync(host, dense, sizeof(float) * (size_t)g.n,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host, dense, sizeof(float) * (size_t)g.n, h->stream));
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return PE_OK;
 }

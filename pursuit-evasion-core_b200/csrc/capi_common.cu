@@ -1,5 +1,16 @@
 // Library-wide C-ABI entry points: version, last error, launch counter.
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <exception>
+#include <thread>
+
 #include "pe_internal.h"
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
 
 namespace pe {
 
@@ -22,6 +33,50 @@ int cuda_fail(cudaError_t err, const char *what) {
   const int code =
       err == cudaErrorMemoryAllocation ? PE_ENOMEM : PE_ECUDA;
   return fail(code, "%s: %s", what, cudaGetErrorString(err));
+}
+
+namespace {
+
+// Populate the whole pages inside [host, host + bytes) for writing; contents
+// stay.  On a kernel without MADV_POPULATE_WRITE the call fails and the copy
+// takes its faults as it would have.
+void populate_pages(void *host, size_t bytes) {
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t lo = ((uintptr_t)host + page - 1) / page * page;
+  const uintptr_t hi = ((uintptr_t)host + bytes) / page * page;
+  if (hi <= lo) return;
+  auto part = [](uintptr_t a, uintptr_t b) {
+    madvise(reinterpret_cast<void *>(a), b - a, MADV_POPULATE_WRITE);
+  };
+  // about 4 MB per thread (read-back of a 12.6 MB field into a fresh array 3.1 ->
+  // 2.0 ms, of four fields of 43.6 MB 11.5 -> 8.3 ms)
+  const int want = (int)std::min<size_t>(4, (hi - lo) >> 22);
+  std::thread workers[4];
+  int started = 0;
+  const uintptr_t step = (hi - lo) / page / (want > 0 ? want : 1) * page;
+  uintptr_t at = lo;
+  try {
+    for (; started + 1 < want; started++, at += step)
+      workers[started] = std::thread(part, at, at + step);
+  } catch (const std::exception &) {
+    // no more threads: the rest here
+  }
+  part(at, hi);
+  for (int k = 0; k < started; k++) workers[k].join();
+}
+
+}  // namespace
+
+cudaError_t copy_out(void *host, const void *device, size_t bytes, cudaStream_t stream) {
+  if (bytes >= (size_t)1 << 20) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, host) == cudaSuccess) {
+      if (attr.type == cudaMemoryTypeUnregistered) populate_pages(host, bytes);
+    } else {
+      cudaGetLastError();  // (an unknown pointer is the copy's to report)
+    }
+  }
+  return cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, stream);
 }
 
 static std::atomic<int64_t> g_launches{0};

@@ -436,8 +436,7 @@ int pe_relative_copy_field(pe_relative *h, float *host_field) {
   // between steps).
   PE_CUDA_TRY(pe::rel5_pack(h->g, h->a, h->b, h->stream));
   pe::count_launches(1);
-  PE_CUDA_TRY(cudaMemcpyAsync(host_field, h->b, sizeof(float) * (size_t)h->g.n,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_field, h->b, sizeof(float) * (size_t)h->g.n, h->stream));
   return read_stats(h);
 }
 
@@ -447,8 +446,7 @@ int pe_relative_copy_arrival(pe_relative *h, float *host_arrival) {
   if (!host_arrival) return fail(PE_EINVAL, "host_arrival is NULL");
   PE_CUDA_TRY(pe::rel5_pack(h->g, h->arrival, h->b, h->stream));
   pe::count_launches(1);
-  PE_CUDA_TRY(cudaMemcpyAsync(host_arrival, h->b, sizeof(float) * (size_t)h->g.n,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_arrival, h->b, sizeof(float) * (size_t)h->g.n, h->stream));
   return read_stats(h);
 }
 

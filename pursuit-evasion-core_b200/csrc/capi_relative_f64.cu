@@ -223,8 +223,7 @@ int pe_relative_f64_copy_field(pe_relative_f64 *h, double *host_dst) {
   if (rc) return rc;
   if (!host_dst) return fail(PE_EINVAL, "host_dst is NULL");
   if (!h->initialized) return fail(PE_ESTATE, "copy before init");
-  PE_CUDA_TRY(cudaMemcpyAsync(host_dst, h->a, sizeof(double) * (size_t)h->g.n,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_dst, h->a, sizeof(double) * (size_t)h->g.n, h->stream));
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   pe::Rel5Stats host{};
   return read_stats(h, &host);

@@ -511,8 +511,7 @@ int pe_semilag_copy_value(pe_semilag *h, float *host_value) {
   int rc = enter(h);
   if (rc) return rc;
   if (!host_value) return fail(PE_EINVAL, "host_value is NULL");
-  PE_CUDA_TRY(cudaMemcpyAsync(host_value, h->a, sizeof(float) * (size_t)h->g.n,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_value, h->a, sizeof(float) * (size_t)h->g.n, h->stream));
   return read_stats(h);
 }
 
@@ -531,11 +530,9 @@ int pe_semilag_copy_policy(pe_semilag *h, uint8_t *host_p, uint8_t *host_e) {
   if (!h->policy_valid)
     return fail(PE_ESTATE, "no policy: run pe_semilag_backup(h, 1) first");
   if (host_p)
-    PE_CUDA_TRY(cudaMemcpyAsync(host_p, h->pol_p, (size_t)h->g.n,
-                                cudaMemcpyDeviceToHost, h->stream));
+    PE_CUDA_TRY(pe::copy_out(host_p, h->pol_p, (size_t)h->g.n, h->stream));
   if (host_e)
-    PE_CUDA_TRY(cudaMemcpyAsync(host_e, h->pol_e, (size_t)h->g.n,
-                                cudaMemcpyDeviceToHost, h->stream));
+    PE_CUDA_TRY(pe::copy_out(host_e, h->pol_e, (size_t)h->g.n, h->stream));
   return read_stats(h);
 }
 
@@ -640,8 +637,8 @@ int pe_semilag_copy_arrival(pe_semilag *h, float *host_arrival) {
   if (rc) return rc;
   if (!host_arrival) return fail(PE_EINVAL, "host_arrival is NULL");
   if (!h->arrival) return fail(PE_ESTATE, "arrival is not tracked");
-  PE_CUDA_TRY(cudaMemcpyAsync(host_arrival, h->arrival, sizeof(float) * (size_t)h->g.n,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_arrival, h->arrival, sizeof(float) * (size_t)h->g.n,
+                           h->stream));
   PE_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return PE_OK;
 }

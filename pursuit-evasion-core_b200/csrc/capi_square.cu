@@ -285,8 +285,7 @@ int pe_square_copy_field(pe_square *h, float *host_field) {
   int rc = enter(h);
   if (rc) return rc;
   if (!host_field) return fail(PE_EINVAL, "host_field is NULL");
-  PE_CUDA_TRY(cudaMemcpyAsync(host_field, h->a, sizeof(float) * (size_t)h->g.cells,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_field, h->a, sizeof(float) * (size_t)h->g.cells, h->stream));
   return read_stats(h);
 }
 
@@ -294,8 +293,8 @@ int pe_square_copy_arrival(pe_square *h, float *host_arrival) {
   int rc = enter(h);
   if (rc) return rc;
   if (!host_arrival) return fail(PE_EINVAL, "host_arrival is NULL");
-  PE_CUDA_TRY(cudaMemcpyAsync(host_arrival, h->arrival, sizeof(float) * (size_t)h->g.cells,
-                              cudaMemcpyDeviceToHost, h->stream));
+  PE_CUDA_TRY(pe::copy_out(host_arrival, h->arrival, sizeof(float) * (size_t)h->g.cells,
+                           h->stream));
   return read_stats(h);
 }
 

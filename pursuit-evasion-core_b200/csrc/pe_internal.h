@@ -26,6 +26,12 @@ int cuda_fail(cudaError_t err, const char *what);
 // Count of kernels this library has launched (pe_launch_count()).
 void count_launches(int64_t n);
 
+// Asynchronous device-to-host copy of a result.  Large pageable destinations
+// (a fresh array's pages do not exist yet) are populated first, in parallel and
+// while the device may still be computing, instead of page by page inside the
+// copy.
+cudaError_t copy_out(void *host, const void *device, size_t bytes, cudaStream_t stream);
+
 // Per-launch device time from CUDA event pairs recorded on the launching
 // stream, summed per slot (e.g. RK2 stage 1 / stage 2).  Finished pairs are
 // harvested without blocking once many are outstanding, so profiling adds
