@@ -45,11 +45,15 @@ void populate_pages(void *host, size_t bytes) {
   const uintptr_t lo = ((uintptr_t)host + page - 1) / page * page;
   const uintptr_t hi = ((uintptr_t)host + bytes) / page * page;
   if (hi <= lo) return;
+  // Memory that the allocator hands out again is resident already: a walk over
+  // it would only cost time (12.6 MB in reused pages: 0.72 ms with, 0.66 without;
+  // 77.8 MB in a fresh mapping: 7.3 ms with, 16.4 without).  The last page tells.
+  unsigned char resident = 0;
+  if (mincore(reinterpret_cast<void *>(hi - page), page, &resident) == 0 && (resident & 1)) return;
   auto part = [](uintptr_t a, uintptr_t b) {
     madvise(reinterpret_cast<void *>(a), b - a, MADV_POPULATE_WRITE);
   };
-  // about 4 MB per thread (read-back of a 12.6 MB field into a fresh array 3.1 ->
-  // 2.0 ms, of four fields of 43.6 MB 11.5 -> 8.3 ms)
+  // about 4 MB per thread
   const int want = (int)std::min<size_t>(4, (hi - lo) >> 22);
   std::thread workers[4];
   int started = 0;
