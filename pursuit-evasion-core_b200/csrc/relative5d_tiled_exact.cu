@@ -204,8 +204,11 @@ cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t 
 // The tiled kernel takes the padded layout on 16-byte bounds, in a tile whose
 // rings and tables fit, where it is the faster one: its stage takes about 3.4
 // times the float32 stage's, the thread-per-cell stage 4 us and 45 us per
-// million cells (B200: 17x12x7x7 39 against 29 us per RK2 step, 21x16x9x9 63
-// against 66, 33x24x11x11 199 against 293, 65x48x21x21 3550 against 8000).
+// million cells, row padding not counted.  Near equal estimates the tiled one is
+// up to 17 % low, so it has to be 8 % below (B200, us per RK2 step in tiles and
+// per cell: 21x16x7x7 42.7, 38.1; 21x16x9x9 60.2, 59.0; 25x18x7x7 65.1, 53.2;
+// 25x18x9x9 64, 88; 33x24x11x11 207, 293; 65x48x21x21 3600, 8000.  It costs
+// 23x16x7x7 44.7, 46.7).
 bool rel5_walk_exact_applies(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s) {
   if (g.xp % 4 != 0 || g.sy != g.xp ||
       ((reinterpret_cast<uintptr_t>(s.src) | reinterpret_cast<uintptr_t>(s.dst)) & 15) != 0)
@@ -213,8 +216,9 @@ bool rel5_walk_exact_applies(const Rel5Grid &g, const Rel5Tile &t, const Rel5Sta
   if (!rel5_tile_valid(g, t) ||
       smem_layout(t.rows, g.xp, table_bytes(g)).bytes > 227 * 1024)
     return false;
-  const double cells = (double)g.se * g.nve * (g.own_n > 0 ? g.own_n : g.nvp);
-  return 3.4 * rel5_tile_cost(g, t) < 4.0 + 45e-6 * cells;
+  const double cells =
+      (double)g.nx * g.nx * g.nh * g.nve * (g.own_n > 0 ? g.own_n : g.nvp);
+  return 3.4 * rel5_tile_cost(g, t) < 0.92 * (4.0 + 45e-6 * cells);
 }
 
 cudaError_t rel5_stage_f64_tiled(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s,
