@@ -14,21 +14,31 @@
 // under the other's epilogue, which is the bound: SiLU takes two special
 // function operations (four clocks of an SM's unit per warp) and about 9
 // instructions per element.  Training
-// (TPC = 1) also writes each layer's pre-activation and activation; inference
+// (TPC = 1) also writes each layer's pre-activation and activation (below); inference
 // writes the 128 outputs of a tile and can make its own input features, so
 // nothing of a row but its output touches memory.
 //
 // Measured: 8.5 M grid nodes (41x30x13x13) 45.7 ms with a launch per layer,
 // 10.7 ms with this kernel and the division of the C expression, 6.7 ms with
-// the packed SiLU; a query of 1000 states 116 -> 25 us.  A training step at
-// 8192 rows (64 CTAs, one tile each, the chain of layers its latency): forward
-// 145 -> 43 us, backward with the weight gradients 400 -> 67 us.
+// the packed SiLU; a query of 1000 states 116 -> 25 us.
 //
 // Backward (per 128-row tile): dz of the last layer from the head, then
-// dz_{l-1} = (dz_l W_l) silu'(z_{l-1}) down the layers, with the bias and head
-// gradients summed on the way.  Weight gradients: dW_l = dz_l^T prev_l over
-// the rows, both operands as they lie in memory (MN-major tiles), the rows
-// split over the CTAs, partial sums added with 16-byte atomics.
+// dz_{l-1} = (dz_l W_l) silu'(z_{l-1}) down the layers, with the head gradients
+// summed on the way.  Weight gradients: dW_l = dz_l^T prev_l over the rows,
+// both operands as they lie in memory (MN-major tiles), the rows split over the
+// CTAs, partial sums added with 16-byte atomics; the bias gradients are column
+// sums of the same dz tiles.
+//
+// A training batch of 8192 rows is 64 tiles for 148 SMs and each tile a chain
+// of layers, so a training pass's time is that chain: MMA, epilogue, MMA, ..
+// Two CTAs of a cluster share a tile: each takes 128 columns of every layer
+// and writes its half of the next operand into both CTAs' shared memory.  The
+// epilogue hands the tile to the next MMAs before it writes z, h or dz to
+// memory, in whole rows (z by TMA from a staged block per warp, and one layer
+// ahead by TMA in the backward pass): with a row per lane and before the
+// hand-over those stores were 6,000 of a layer's 16,000 clocks.  A step at 8192
+// rows, launch per layer, then one CTA per tile, then this: forward 145, 43,
+// 34 us; backward with all gradients 400, 66, 40 us.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets the error flag
 // of pe_mlp_gemm_tc_timeouts and the CTA still releases its tensor memory.
@@ -53,7 +63,7 @@ constexpr int W_SLICE = H * 128;    // 64 K columns of 256 weight rows, bytes
 enum Input { FEATURES = 0, RELATIVE_NODES = 1, RELATIVE_STATES = 2, WORLD_NODES = 3 };
 
 struct ForwardArgs {
-  CUtensorMap w[MAX_LAYERS], feat;
+  CUtensorMap w[MAX_LAYERS], feat, zmap[MAX_LAYERS];
   int layers, rows, groups;
   const float *bias[MAX_LAYERS], *w_out, *b_out;
   float *z[MAX_LAYERS];          // training: pre-activations [rows][256]
@@ -69,17 +79,18 @@ struct ForwardArgs {
 
 struct BackwardArgs {
   CUtensorMap wt[MAX_LAYERS];  // transposed weights [in][out]
+  CUtensorMap zmap[MAX_LAYERS];
   int layers;
-  const float *z[MAX_LAYERS], *dy, *w_out;
+  const float *dy, *w_out;
   const __nv_bfloat16 *h_last;
   __nv_bfloat16 *dz[MAX_LAYERS];
-  float *gb[MAX_LAYERS], *gw_out, *gb_out;
+  float *gw_out, *gb_out;
   unsigned *error;
 };
 
 struct WeightGradArgs {
   CUtensorMap dz[MAX_LAYERS], prev[MAX_LAYERS];
-  float *gw[MAX_LAYERS];
+  float *gw[MAX_LAYERS], *gb[MAX_LAYERS];
   int width0;  // input columns of layer 0 (128 or 256)
   int ksteps;  // 64-row steps over all rows
   unsigned *error;
@@ -113,6 +124,82 @@ __device__ __forceinline__ void fence_after() {
 }
 __device__ __forceinline__ void fence_async_shared() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// --- a cluster of two CTAs on one tile (CL = 2): each takes 128 of the 256
+// columns of every layer and writes its half of the next operand into both
+// CTAs' shared memory.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t peer_addr(const void *p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// bounded wait that also acquires what the peer CTA released
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity,
+                                                  unsigned *error) {
+  for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n"
+        " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  atomicOr(error, 1u);
+  return false;
+}
+template <int CL>
+__device__ __forceinline__ bool tile_wait(uint64_t *bar, uint32_t parity, unsigned *error) {
+  return CL == 2 ? mbar_wait_cluster(bar, parity, error) : mbar_wait(bar, parity, error);
+}
+// the same by a whole warp, one answer for all lanes (the warp-wide operations
+// that follow need them together also after a wait that gave up)
+template <int CL>
+__device__ __forceinline__ bool tile_wait_warp(uint64_t *bar, uint32_t parity, unsigned *error) {
+  return __all_sync(0xffffffffu, tile_wait<CL>(bar, parity, error)) != 0;
+}
+// A warp's part of the tile is written: the tensor core (async proxy) of every
+// CTA of the cluster may read it.
+template <int CL>
+__device__ __forceinline__ void tile_arrive(uint64_t *bar, uint32_t rank) {
+  if (CL == 1) {
+    fence_async_shared();
+    mbar_arrive(bar);
+    return;
+  }
+  asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
+  __syncwarp();
+  if ((threadIdx.x & 31) < CL)
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                     peer_addr(bar, threadIdx.x & 31))
+                 : "memory");
+}
+// arrivals per phase of a tile barrier that `warps` warps a CTA complete
+template <int CL>
+__host__ __device__ constexpr int tile_arrivals(int warps) { return CL == 1 ? 32 * warps : CL * warps; }
+// the issued MMAs are done reading the tile, told to every CTA that writes it
+template <int CL>
+__device__ __forceinline__ void acc_commit(uint64_t *bar) {
+  if (CL == 1)
+    mma_commit(bar);
+  else
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster"
+        ".b64 [%0], %1;" ::"r"(smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t r[32], uint32_t taddr) {
@@ -190,13 +277,6 @@ __device__ __forceinline__ void st_global32(void *p, const uint32_t v[8]) {
                "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
-__device__ __forceinline__ void ld_global32(uint32_t v[8], const void *p) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
-                 "=r"(v[6]), "=r"(v[7])
-               : "l"(p));
-}
-
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&p);
@@ -217,22 +297,59 @@ __device__ __forceinline__ void store_tile32(uint8_t *tile, int r, int c0, const
     *reinterpret_cast<uint4 *>(tile + unit_off(r, c0 / 8 + k)) =
         make_uint4(p[4 * k], p[4 * k + 1], p[4 * k + 2], p[4 * k + 3]);
 }
+// the same into the peer's tile
+__device__ __forceinline__ void store_peer32(uint32_t tile, int r, int c0, const uint32_t p[16]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                     tile + unit_off(r, c0 / 8 + k)),
+                 "r"(p[4 * k]), "r"(p[4 * k + 1]), "r"(p[4 * k + 2]), "r"(p[4 * k + 3])
+                 : "memory");
+}
 
-template <int TPC>
+// 32 columns from c0 of 32 rows from r0 of the tile to a [rows][256] array,
+// four lanes a row (whole sectors; a lane a row took 62 clocks an instruction)
+__device__ __forceinline__ void write_out32(__nv_bfloat16 *out, int64_t row0, const uint8_t *tile,
+                                            int r0, int c0, int lane) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int r = r0 + 8 * i + lane / 4, u = c0 / 8 + lane % 4;
+    *reinterpret_cast<uint4 *>(out + (row0 + r) * H + 8 * u) =
+        *reinterpret_cast<const uint4 *>(tile + unit_off(r, u));
+  }
+}
+// A warp's 32 x 32 block of z in shared memory: the 128B-swizzled box of zmap.
+constexpr int Z_BLOCK = 32 * 32 * 4;
+__device__ __forceinline__ int z_unit(int r, int u) { return r * 128 + ((u ^ (r & 7)) << 4); }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int y,
+                                             const void *src) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+          reinterpret_cast<uint64_t>(map)),
+      "r"(x), "r"(y), "r"(smem_u32(src))
+      : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+template <int TPC, int CL>
 struct ForwardLayout {
   static constexpr int STAGES = TPC == 2 ? 2 : 4;
   static constexpr int W = TPC * A_TILE;
-  static constexpr int BIAS = W + STAGES * W_SLICE;  // [layers][256], then w_out
+  static constexpr int Z = W + STAGES * W_SLICE / CL;  // (CL = 2) a block per warp
+  static constexpr int BIAS = Z + (CL == 2 ? EW * Z_BLOCK : 0);  // [layers][256], then w_out
   static constexpr int BARS = BIAS + (MAX_LAYERS + 1) * H * 4;
   static constexpr int BYTES = BARS + 8 * (2 * STAGES + 3 * TPC) + 16;
 };
 
-template <int TPC, int INPUT, bool TRAIN>
+template <int TPC, int INPUT, bool TRAIN, int CL>
 __global__ void __launch_bounds__(THREADS, 1)
     forward_kernel(const __grid_constant__ ForwardArgs g) {
-  using L = ForwardLayout<TPC>;
+  using L = ForwardLayout<TPC, CL>;
+  static_assert(CL == 1 || (TPC == 1 && TRAIN && INPUT == FEATURES), "");
   constexpr int WPT = EW / TPC;        // epilogue warps of a tile
-  constexpr int COLS = H * 4 / WPT;    // columns of one warp
+  constexpr int N = H / CL;            // columns of this CTA
+  constexpr int COLS = N * 4 / WPT;    // columns of one warp
+  constexpr int SLICE = W_SLICE / CL;
   constexpr int S = L::STAGES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = reinterpret_cast<uint8_t *>(
@@ -245,6 +362,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint64_t *f_full = acc_full + TPC;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(f_full + TPC);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = CL == 1 ? 0 : cluster_rank();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
@@ -252,8 +370,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_init(&w_empty[s], 1);
     }
     for (int t = 0; t < TPC; t++) {
-      mbar_init(&a_ready[t], 32 * WPT);
-      mbar_init(&acc_full[t], 1);
+      mbar_init(&a_ready[t], tile_arrivals<CL>(WPT));
+      mbar_init(&acc_full[t], CL);
       mbar_init(&f_full[t], 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -261,7 +379,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == EW + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(TPC * H)
+                 "r"(TPC * N)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -270,6 +388,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   for (int i = threadIdx.x; i < H; i += THREADS) wout[i] = g.w_out[i];
   fence_before();
   __syncthreads();
+  if (CL == 2) cluster_sync();  // the peer's barriers are initialised
   fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -281,7 +400,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {
       bool ok = true;
       unsigned n = 0;  // slices issued
-      for (int grp = blockIdx.x; grp < g.groups && ok; grp += gridDim.x) {
+      for (int grp = blockIdx.x / CL; grp < g.groups && ok; grp += gridDim.x / CL) {
         if (INPUT == FEATURES)
           for (int t = 0; t < TPC; t++) {
             mbar_expect_tx(&f_full[t], 2 * A_CHUNK);
@@ -295,8 +414,8 @@ __global__ void __launch_bounds__(THREADS, 1)
               const int s = n % S;
               if (n >= S) ok = mbar_wait(&w_empty[s], ((n / S) - 1) & 1, g.error);
               if (!ok) break;
-              mbar_expect_tx(&w_full[s], W_SLICE);
-              tma_load_2d(sW + s * W_SLICE, &g.w[l], k * TK, 0, &w_full[s]);
+              mbar_expect_tx(&w_full[s], SLICE);
+              tma_load_2d(sW + s * SLICE, &g.w[l], k * TK, (int)rank * N, &w_full[s]);
               n++;
             }
       }
@@ -308,13 +427,14 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   } else if (warp == EW + 1) {  // ---- MMA issuer
     if (lane == 0) {
-      constexpr uint32_t ID = instr_desc(H, false);
+      constexpr uint32_t ID = instr_desc(N, false);
       bool ok = true;
       unsigned n = 0, pass = 0;
-      for (int grp = blockIdx.x; grp < g.groups && ok; grp += gridDim.x)
+      for (int grp = blockIdx.x / CL; grp < g.groups && ok; grp += gridDim.x / CL)
         for (int l = 0; l < g.layers && ok; l++, pass++)
           for (int t = 0; t < TPC && ok; t++) {
-            ok = mbar_wait(&a_ready[t], pass & 1, g.error);
+            ok = tile_wait<CL>(&a_ready[t], pass & 1, g.error);
+            if (CL == 2) asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
             if (ok && INPUT == FEATURES && l == 0) ok = mbar_wait(&f_full[t], 0, g.error);
             for (int k = 0; k < slices(l) && ok; k++, n++) {
               const int s = n % S;
@@ -322,26 +442,28 @@ __global__ void __launch_bounds__(THREADS, 1)
               if (!ok) break;
               fence_after();
               const uint32_t a0 = smem_u32(sA + t * A_TILE + k * A_CHUNK);
-              const uint32_t b0 = smem_u32(sW + s * W_SLICE);
+              const uint32_t b0 = smem_u32(sW + s * SLICE);
               const int steps = INPUT != FEATURES && l == 0 ? 1 : TK / 16;
               for (int kk = 0; kk < steps; kk++)
-                mma256(tmem + t * H, smem_desc_sw128(a0 + kk * 32),
+                mma256(tmem + t * N, smem_desc_sw128(a0 + kk * 32),
                        smem_desc_sw128(b0 + kk * 32), ID, (k | kk) != 0);
               mma_commit(&w_empty[s]);
             }
-            mma_commit(&acc_full[t]);  // (also after a wait that gave up)
+            acc_commit<CL>(&acc_full[t]);  // (also after a wait that gave up)
           }
     }
   } else {  // ---- epilogues
     const int t = warp / WPT, part = (warp % WPT) / 4, quarter = warp & 3;
     const int r = quarter * 32 + lane;   // row in the tile
-    const int col0 = part * COLS;
+    const int col0 = (int)rank * N + part * COLS;
     uint8_t *tile = sA + t * A_TILE;
-    const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + t * H + col0;
+    const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + t * N + part * COLS;
+    const uint32_t peer = CL == 1 ? 0 : peer_addr(tile, rank ^ 1);
+    uint8_t *zblock = base + L::Z + warp * Z_BLOCK;  // (CL = 2)
     bool ok = true;  // after a wait that gave up every warp still meets every barrier
     unsigned pass = 0;
     float sq = 0.f;
-    for (int grp = blockIdx.x; grp < g.groups; grp += gridDim.x) {
+    for (int grp = blockIdx.x / CL; grp < g.groups; grp += gridDim.x / CL) {
       const int64_t row = (int64_t)(grp * TPC + t) * TM + r;
       if (INPUT != FEATURES && part == 0) {
         float v[kMaxFeatures] = {};
@@ -356,10 +478,14 @@ __global__ void __launch_bounds__(THREADS, 1)
         *reinterpret_cast<uint4 *>(tile + unit_off(r, 0)) = pack_features(v);
         *reinterpret_cast<uint4 *>(tile + unit_off(r, 1)) = pack_features(v + 8);
       }
-      fence_async_shared();
-      mbar_arrive(&a_ready[t]);
+      tile_arrive<CL>(&a_ready[t], rank);
       for (int l = 0; l < g.layers; l++, pass++) {
-        if (ok) ok = mbar_wait(&acc_full[t], pass & 1, g.error);
+        // (one answer per warp for the warp-wide hand-over of a training pass;
+        // inference has none and does without the vote, 6.70 against 6.87 ms for
+        // 8.5 M nodes)
+        if (ok)
+          ok = TRAIN ? tile_wait_warp<CL>(&acc_full[t], pass & 1, g.error)
+                     : mbar_wait(&acc_full[t], pass & 1, g.error);
         if (!ok) continue;
         fence_after();
         const bool last = l == g.layers - 1;
@@ -388,29 +514,48 @@ __global__ void __launch_bounds__(THREADS, 1)
               a[k + 3] = __float_as_uint(z1.y);
             }
           }
-          if (TRAIN) {
+          if (TRAIN && CL == 1) {
             if (g.z[l])
               for (int k = 0; k < 4; k++) st_global32(g.z[l] + row * H + col0 + c0 + 8 * k, a + 8 * k);
             for (int k = 0; k < 2; k++)
               st_global32(g.h[l] + row * H + col0 + c0 + 16 * k, p + 8 * k);
           }
           store_tile32(tile, r, col0 + c0, p);
+          if (CL == 2) {
+            // the next layer starts on the tile first; z and h leave under it
+            store_peer32(peer, r, col0, p);
+            fence_before();
+            tile_arrive<CL>(&a_ready[t], rank);
+            if (g.z[l]) {
+              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < 8; u++)
+                *reinterpret_cast<uint4 *>(zblock + z_unit(lane, u)) =
+                    make_uint4(a[4 * u], a[4 * u + 1], a[4 * u + 2], a[4 * u + 3]);
+              fence_async_shared();
+              __syncwarp();
+              if (lane == 0) tma_store_2d(&g.zmap[l], col0, (int)row - lane, zblock);
+            }
+            write_out32(g.h[l], row - r, tile, quarter * 32, col0, lane);
+          }
         }
-        fence_before();
-        if (!last) {
-          fence_async_shared();
-          mbar_arrive(&a_ready[t]);
+        if (CL == 1) {
+          fence_before();
+          if (!last) tile_arrive<CL>(&a_ready[t], rank);
         }
       }
-      // the head, a warp per row: lane l sums columns l, l + 32, ..
+      // the head, a warp per row: lane l sums columns l, l + 32, ..; a cluster's
+      // CTAs take half of the rows each, once both halves of the columns are in
+      if (CL == 2 && ok) ok = tile_wait_warp<CL>(&a_ready[t], pass & 1, g.error);
       asm volatile("bar.sync %0, %1;" ::"r"(1 + t), "n"(32 * WPT) : "memory");
       float w[H / 32];
 #pragma unroll
       for (int i = 0; i < H / 32; i++) w[i] = wout[lane + 32 * i];
       const float b_out = g.b_out[0];
 #pragma unroll 4
-      for (int q = 0; q < TM / WPT; q++) {
-        const int rr = (warp % WPT) * (TM / WPT) + q;
+      for (int q = 0; q < TM / CL / WPT; q++) {
+        const int rr = (int)rank * (TM / CL) + (warp % WPT) * (TM / CL / WPT) + q;
         float sum = 0.f;
 #pragma unroll
         for (int i = 0; i < H / 32; i++) {
@@ -434,56 +579,69 @@ __global__ void __launch_bounds__(THREADS, 1)
       asm volatile("bar.sync %0, %1;" ::"r"(1 + t), "n"(32 * WPT) : "memory");
     }
     if (TRAIN && g.target && lane == 0) atomicAdd(g.loss, sq);
+    if (CL == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncwarp();
   fence_before();
   __syncthreads();
+  if (CL == 2) cluster_sync();  // the peer is done with this shared memory
   if (warp == EW + 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(TPC * H)
+                 "r"(TPC * N)
                  : "memory");
 }
 
 // ------------------------------------------------------------- backward
+constexpr int BCL = 2;  // CTAs per tile, always
 struct BackwardLayout {
   static constexpr int STAGES = 4;
   static constexpr int W = A_TILE;
-  static constexpr int WOUT = W + STAGES * W_SLICE;
+  static constexpr int Z = W + STAGES * W_SLICE / BCL;  // a block per warp
+  static constexpr int WOUT = Z + EW * Z_BLOCK;
   static constexpr int DY = WOUT + H * 4;
-  static constexpr int BARS = DY + TM * 4;
-  static constexpr int BYTES = BARS + 8 * (2 * STAGES + 2) + 16;
+  static constexpr int RED = DY + TM * 4;  // [8 ranges][128] partial column sums
+  static constexpr int BARS = RED + 4 * H * 4;
+  static constexpr int BYTES = BARS + 8 * (2 * STAGES + 2 + EW) + 16;
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
     backward_kernel(const __grid_constant__ BackwardArgs g) {
   using L = BackwardLayout;
+  constexpr int CL = BCL;
   constexpr int S = L::STAGES;
-  constexpr int COLS = 64;  // columns of one epilogue warp
+  constexpr int N = H / CL;     // columns of this CTA
+  constexpr int COLS = N / 4;   // columns of one epilogue warp
+  static_assert(COLS == 32, "a warp takes one 32 x 32 block");
+  constexpr int SLICE = W_SLICE / CL;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *tile = base, *sW = base + L::W;
   float *wout = reinterpret_cast<float *>(base + L::WOUT);
   float *dys = reinterpret_cast<float *>(base + L::DY);
+  float *red = reinterpret_cast<float *>(base + L::RED);
   uint64_t *w_full = reinterpret_cast<uint64_t *>(base + L::BARS);
   uint64_t *w_empty = w_full + S, *a_ready = w_empty + S, *acc_full = a_ready + 1;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+  uint64_t *z_full = acc_full + 1;  // one per epilogue warp
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(z_full + EW);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row0 = (int64_t)blockIdx.x * TM;
+  const uint32_t rank = cluster_rank();
+  const int64_t row0 = (int64_t)(blockIdx.x / CL) * TM;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
       mbar_init(&w_full[s], 1);
       mbar_init(&w_empty[s], 1);
     }
-    mbar_init(a_ready, 32 * EW);
-    mbar_init(acc_full, 1);
+    mbar_init(a_ready, tile_arrivals<CL>(EW));
+    mbar_init(acc_full, CL);
+    for (int w = 0; w < EW; w++) mbar_init(&z_full[w], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == EW + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(H)
+                 "r"(N)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -491,6 +649,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   for (int i = threadIdx.x; i < TM; i += THREADS) dys[i] = g.dy[row0 + i];
   fence_before();
   __syncthreads();
+  cluster_sync();  // the peer's barriers are initialised
   fence_after();
   const uint32_t tmem = *tmem_slot;
 
@@ -503,112 +662,124 @@ __global__ void __launch_bounds__(THREADS, 1)
           const int s = n % S;
           if (n >= S) ok = mbar_wait(&w_empty[s], ((n / S) - 1) & 1, g.error);
           if (!ok) break;
-          mbar_expect_tx(&w_full[s], W_SLICE);
-          tma_load_2d(sW + s * W_SLICE, &g.wt[l], k * TK, 0, &w_full[s]);
+          mbar_expect_tx(&w_full[s], SLICE);
+          tma_load_2d(sW + s * SLICE, &g.wt[l], k * TK, (int)rank * N, &w_full[s]);
         }
       for (unsigned k = n > S ? n - S : 0; k < n; k++)
         mbar_wait(&w_full[k % S], (k / S) & 1, g.error);
     }
   } else if (warp == EW + 1) {
     if (lane == 0) {
-      constexpr uint32_t ID = instr_desc(H, false);
+      constexpr uint32_t ID = instr_desc(N, false);
       bool ok = true;
       unsigned n = 0, pass = 0;
       for (int l = g.layers - 1; l > 0 && ok; l--, pass++) {
-        ok = mbar_wait(a_ready, pass & 1, g.error);
+        ok = tile_wait<CL>(a_ready, pass & 1, g.error);
+        asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
         for (int k = 0; k < 4 && ok; k++, n++) {
           const int s = n % S;
           ok = mbar_wait(&w_full[s], (n / S) & 1, g.error);
           if (!ok) break;
           fence_after();
           const uint32_t a0 = smem_u32(tile + k * A_CHUNK);
-          const uint32_t b0 = smem_u32(sW + s * W_SLICE);
+          const uint32_t b0 = smem_u32(sW + s * SLICE);
           for (int kk = 0; kk < TK / 16; kk++)
             mma256(tmem, smem_desc_sw128(a0 + kk * 32), smem_desc_sw128(b0 + kk * 32), ID,
                    (k | kk) != 0);
           mma_commit(&w_empty[s]);
         }
-        mma_commit(acc_full);
+        acc_commit<CL>(acc_full);
       }
     }
   } else {
     const int part = warp / 4, quarter = warp & 3;
     const int r = quarter * 32 + lane;
-    const int col0 = part * COLS;
-    const int64_t row = row0 + r;
-    const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
+    const int col0 = (int)rank * N + part * COLS;
+    const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + part * COLS;
+    const uint32_t peer = peer_addr(tile, rank ^ 1);
     const float d = dys[r];
-    // Column pair and row range of the sums: 128 pairs x 4 ranges of 32 rows.
-    const int pair = threadIdx.x & 127, range = threadIdx.x >> 7;
+    // Column pair and row range of the head's sums: this CTA's 64 pairs x 8
+    // ranges of 16 rows.
+    constexpr int ROWS = 32 / CL;
+    const int pair = (int)rank * (N / 2) + threadIdx.x % (N / 2), range = threadIdx.x / (N / 2);
     bool ok = true;
     unsigned pass = 0;
+    // column sums over the tile: the ranges in shared memory first, so that a
+    // CTA adds one partial sum per column
+    auto add_columns = [&](float *out, float v0, float v1) {
+      const int c = 2 * (threadIdx.x % (N / 2));
+      *reinterpret_cast<float2 *>(red + range * N + c) = make_float2(v0, v1);
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
+      if (threadIdx.x >= N || !ok) return;
+      float part[4 * CL];
+#pragma unroll
+      for (int i = 0; i < 4 * CL; i++) part[i] = red[i * N + threadIdx.x];
+#pragma unroll
+      for (int w = 2 * CL; w > 0; w /= 2)
+#pragma unroll
+        for (int i = 0; i < w; i++) part[i] += part[i + w];
+      atomicAdd(out + (int)rank * N + threadIdx.x, part[0]);
+    };
+    // z of the next layer down arrives while this one is worked on
+    uint8_t *zblock = base + L::Z + warp * Z_BLOCK;
+    auto load_z = [&](int l) {
+      if (lane != 0) return;
+      fence_async_shared();  // the block's reads come before the copy
+      mbar_expect_tx(&z_full[warp], Z_BLOCK);
+      tma_load_2d(zblock, &g.zmap[l], col0, (int)row0 + quarter * 32, &z_full[warp]);
+    };
+    bool z_asked = true;
+    load_z(g.layers - 1);
     for (int l = g.layers - 1; l >= 0; l--) {
       const bool head = l == g.layers - 1;
       uint32_t zr[32];
-      const float *zp = g.z[l] + row * H + col0;
-      for (int k = 0; k < 4; k++) ld_global32(zr + 8 * k, zp + 8 * k);
+      // (a copy is asked for only while no wait has given up, and always
+      // waited for: none is in flight when the CTA leaves)
+      if (z_asked) ok = tile_wait_warp<1>(&z_full[warp], (g.layers - 1 - l) & 1, g.error) && ok;
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        *reinterpret_cast<uint4 *>(zr + 4 * u) =
+            *reinterpret_cast<const uint4 *>(zblock + z_unit(lane, u));
+      __syncwarp();
+      z_asked = ok && l > 0;
+      if (z_asked) load_z(l - 1);
       if (!head) {
-        if (ok) ok = mbar_wait(acc_full, pass & 1, g.error);
+        if (ok) ok = tile_wait_warp<CL>(acc_full, pass & 1, g.error);
         pass++;
         fence_after();
-        // the column sums of the previous dz have been read out of the tile
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
       }
-#pragma unroll 1
-      for (int c0 = 0; c0 < COLS; c0 += 32) {
-        uint32_t a[32], p[16];
-        if (!head) {
-          tmem_ld32(a, acc + c0);
-          tmem_wait();
-        }
+      uint32_t a[32], p[16];
+      if (!head) {
+        tmem_ld32(a, acc);
+        tmem_wait();
+      }
 #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          const float u0 = head ? d * wout[col0 + c0 + k] : __uint_as_float(a[k]);
-          const float u1 = head ? d * wout[col0 + c0 + k + 1] : __uint_as_float(a[k + 1]);
-          const float2 sg = silu_grad2(
-              make_float2(__uint_as_float(zr[k]), __uint_as_float(zr[k + 1])));
-          p[k / 2] = pack2(u0 * sg.x, u1 * sg.y);
-        }
-        if (c0 + 32 < COLS)
-          for (int k = 0; k < 4; k++) ld_global32(zr + 8 * k, zp + c0 + 32 + 8 * k);
-        for (int k = 0; k < 2; k++)
-          st_global32(g.dz[l] + row * H + col0 + c0 + 16 * k, p + 8 * k);
-        store_tile32(tile, r, col0 + c0, p);
+      for (int k = 0; k < 32; k += 2) {
+        const float u0 = head ? d * wout[col0 + k] : __uint_as_float(a[k]);
+        const float u1 = head ? d * wout[col0 + k + 1] : __uint_as_float(a[k + 1]);
+        const float2 sg = silu_grad2(
+            make_float2(__uint_as_float(zr[k]), __uint_as_float(zr[k + 1])));
+        p[k / 2] = pack2(u0 * sg.x, u1 * sg.y);
       }
+      store_tile32(tile, r, col0, p);
+      if (l > 0) store_peer32(peer, r, col0, p);
       fence_before();
-      if (l > 0) {
-        fence_async_shared();
-        mbar_arrive(a_ready);
-      }
-      // bias gradient: column sums of the bf16 dz tile
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
-      float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-      for (int q = 0; q < 32; q++) {
-        const int rr = range * 32 + q;
-        const uint32_t v =
-            *reinterpret_cast<const uint32_t *>(tile + unit_off(rr, pair / 4) + (pair & 3) * 4);
-        s0 += lo16(v);
-        s1 += hi16(v);
-      }
-      if (ok) {
-        atomicAdd(g.gb[l] + 2 * pair, s0);
-        atomicAdd(g.gb[l] + 2 * pair + 1, s1);
-      }
+      if (l > 0) tile_arrive<CL>(a_ready, rank);
+      __syncwarp();
+      write_out32(g.dz[l], row0, tile, quarter * 32, col0, lane);
       if (head) {  // head gradients: dw_out = sum_r dy_r h_r, db_out = sum_r dy_r
         float w0 = 0.f, w1 = 0.f, sd = 0.f;
         const uint32_t *hp =
-            reinterpret_cast<const uint32_t *>(g.h_last + (row0 + range * 32) * H) + pair;
+            reinterpret_cast<const uint32_t *>(g.h_last + (row0 + range * ROWS) * H) + pair;
 #pragma unroll 8
-        for (int q = 0; q < 32; q++) {
+        for (int q = 0; q < ROWS; q++) {
           const uint32_t v = hp[q * (H / 2)];
-          const float dr = dys[range * 32 + q];
+          const float dr = dys[range * ROWS + q];
           w0 = fmaf(dr, lo16(v), w0);
           w1 = fmaf(dr, hi16(v), w1);
           sd += dr;
         }
-        atomicAdd(g.gw_out + 2 * pair, w0);
-        atomicAdd(g.gw_out + 2 * pair + 1, w1);
+        add_columns(g.gw_out, w0, w1);
         if (pair == 0) atomicAdd(g.gb_out, sd);
       }
     }
@@ -616,8 +787,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncwarp();
   fence_before();
   __syncthreads();
+  cluster_sync();  // the peer is done with this shared memory
   if (warp == EW + 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(H)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(N)
                  : "memory");
 }
 
@@ -660,7 +832,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < G_STAGES; s++) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+      mbar_init(&empty[s], 1 + G_WARPS);  // the MMAs, and each summing warp
     }
     mbar_init(done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -717,8 +889,43 @@ __global__ void __launch_bounds__(G_THREADS, 1)
       mma_commit(done);
     }
   } else {
+    // Bias gradients: the column sums of the dz tiles while the MMAs read them
+    // (64 column pairs x 4 groups of 16 rows a stage).  Here a column takes
+    // one partial sum per row split (18 at 8192 rows), against one per 128-row
+    // tile where dz is made, and off that kernel's chain of layers.
+    const int pair = threadIdx.x & 63, group = threadIdx.x >> 6;
+    float s0 = 0.f, s1 = 0.f;
+    bool summed = true;
+    for (int n = 0; n < k1 - k0; n++) {
+      const int s = n % G_STAGES;
+      summed = tile_wait_warp<1>(&full[s], (n / G_STAGES) & 1, g.error);
+      if (!summed) break;
+      const uint8_t *block = base + s * G_STAGE + (pair >> 5) * G_BLOCK + (pair & 3) * 4;
+      float t0 = 0.f, t1 = 0.f;
+#pragma unroll
+      for (int q = 0; q < 16; q++) {
+        const int r = group * 16 + q, u = (pair & 31) >> 2;
+        const uint32_t v =
+            *reinterpret_cast<const uint32_t *>(block + r * 128 + ((u ^ (r & 7)) << 4));
+        t0 += lo16(v);
+        t1 += hi16(v);
+      }
+      s0 += t0;
+      s1 += t1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
     const bool ok = mbar_wait(done, 0, g.error) && k1 > k0;
     fence_after();
+    // every warp is done with the ring: its space is free for what follows
+    float *sums = reinterpret_cast<float *>(base + 2 * G_STAGE);  // [4][128]
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * G_WARPS) : "memory");
+    *reinterpret_cast<float2 *>(sums + group * TM + 2 * pair) = make_float2(s0, s1);
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * G_WARPS) : "memory");
+    if (threadIdx.x < TM && ok && summed)
+      atomicAdd(g.gb[l] + m0 + threadIdx.x,
+                (sums[threadIdx.x] + sums[TM + threadIdx.x]) +
+                    (sums[2 * TM + threadIdx.x] + sums[3 * TM + threadIdx.x]));
     // warp w: accumulator lanes 32 (w mod 4) .., columns of half w / 4; each
     // 32 x 32 block is turned around in shared memory (the ring is idle now)
     // so that 8 lanes add 128 contiguous bytes of one row
@@ -826,16 +1033,26 @@ int check_net(const pe_mlp_net *n) {
   return PE_OK;
 }
 
-int forward_args(const pe_mlp_net *n, ForwardArgs &g, bool made_features) {
+// z [rows][256] in 128B-swizzled boxes of 32 x 32
+CUresult make_z_map(CUtensorMap *map, const float *z, int rows) {
+  const cuuint64_t dims[2] = {H, (cuuint64_t)rows}, strides[1] = {H * sizeof(float)};
+  const cuuint32_t box[2] = {32, 32}, elem[2] = {1, 1};
+  EncodeTiled encode = encoder();
+  if (!encode) return CUDA_ERROR_NOT_FOUND;
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(z), dims, strides,
+                box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+// cl: CTAs that share the columns of a tile
+int forward_args(const pe_mlp_net *n, ForwardArgs &g, int cl) {
   g.layers = n->layers;
   for (int l = 0; l < n->layers; l++) {
     const int K = l == 0 ? n->in_width : H;
-    // made features: the 64-column slice of which 16 are used
-    if (make_map(&g.w[l], n->w16[l], H, K, K, H) != CUDA_SUCCESS)
+    if (make_map(&g.w[l], n->w16[l], H, K, K, H / cl) != CUDA_SUCCESS)
       return fail(PE_EINVAL, "mlp: tensor map encoding failed");
     g.bias[l] = n->b[l];
   }
-  (void)made_features;
   g.w_out = n->w_out;
   g.b_out = n->b_out;
   g.error = error_word();
@@ -843,24 +1060,46 @@ int forward_args(const pe_mlp_net *n, ForwardArgs &g, bool made_features) {
   return PE_OK;
 }
 
-template <int TPC, int INPUT, bool TRAIN>
-cudaError_t launch_forward(ForwardArgs &g, cudaStream_t stream) {
-  constexpr int bytes = ForwardLayout<TPC>::BYTES + 1024;
-  cudaError_t e = cudaFuncSetAttribute(forward_kernel<TPC, INPUT, TRAIN>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+template <class... P, class... A>
+cudaError_t launch_tiles(void (*kernel)(P...), int grid, int cl, int bytes, cudaStream_t stream,
+                         A &...args) {
+  cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
-  g.groups = (g.rows + TPC * TM - 1) / (TPC * TM);
-  // read features: one group per CTA; made ones: one persistent CTA per SM
-  const int grid = INPUT == FEATURES || g.groups < 148 ? g.groups : 148;
-  forward_kernel<TPC, INPUT, TRAIN><<<grid, THREADS, bytes, stream>>>(g);
-  return cudaGetLastError();
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {(unsigned)cl, 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cl > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+
+template <int TPC, int INPUT, bool TRAIN, int CL = 1>
+cudaError_t launch_forward(ForwardArgs &g, cudaStream_t stream) {
+  g.groups = (g.rows + TPC * TM - 1) / (TPC * TM);
+  // read features: one group per CTA (or cluster); made ones: a persistent CTA per SM
+  const int grid = INPUT == FEATURES || g.groups < 148 ? g.groups : 148;
+  return launch_tiles(forward_kernel<TPC, INPUT, TRAIN, CL>, grid * CL, CL,
+                      ForwardLayout<TPC, CL>::BYTES + 1024, stream, g);
+}
+
+// CTAs per 128-row tile of a forward training pass: two while that many fit the
+// SMs (8192 rows 43.6 us with one, 34.6 with two), one beyond (9600 rows 41.4
+// with one, 64.1 with two, which then take a second wave; 65536: 167 and 240).
+// The backward pass takes two at every size (9600 rows, with the weight
+// gradients, 74 us with one, 72 with two; 19072: 144, 111; 65536: 325, 278).
+inline int cluster_of(int rows) { return 2 * (rows / TM) <= 148 ? 2 : 1; }
 
 // Inference on made features: two tiles per CTA once every SM has two, one
 // (half the latency, twice the CTAs) below that.
 template <int INPUT>
 int infer(const pe_mlp_net *net, ForwardArgs &g, cudaStream_t stream) {
-  int rc = forward_args(net, g, true);
+  int rc = forward_args(net, g, 1);
   if (rc) return rc;
   const cudaError_t e = g.rows > 148 * TM ? launch_forward<2, INPUT, false>(g, stream)
                                           : launch_forward<1, INPUT, false>(g, stream);
@@ -884,7 +1123,8 @@ int pe_mlp_forward(const pe_mlp_net *net, const void *feat, int rows, float *con
       reinterpret_cast<uintptr_t>(feat) % 16)
     return fail(PE_EINVAL, "mlp_forward: rows a multiple of 128, features 16-byte aligned");
   ForwardArgs g{};
-  rc = forward_args(net, g, false);
+  const int cl = cluster_of(rows);
+  rc = forward_args(net, g, cl);
   if (rc) return rc;
   if (tc::make_map(&g.feat, feat, rows, net->in_width, net->in_width, TM) != CUDA_SUCCESS)
     return fail(PE_EINVAL, "mlp_forward: tensor map encoding failed");
@@ -894,14 +1134,17 @@ int pe_mlp_forward(const pe_mlp_net *net, const void *feat, int rows, float *con
     g.h[l] = static_cast<__nv_bfloat16 *>(h[l]);
     if (!g.h[l] || (reinterpret_cast<uintptr_t>(g.h[l]) | reinterpret_cast<uintptr_t>(g.z[l])) % 32)
       return fail(PE_EINVAL, "mlp_forward: activation buffers 32-byte aligned");
+    if (cl == 2 && g.z[l] && make_z_map(&g.zmap[l], g.z[l], rows) != CUDA_SUCCESS)
+      return fail(PE_EINVAL, "mlp_forward: tensor map encoding failed");
   }
   g.target = target;
   g.y = y;
   g.dy = dy;
   g.loss = loss;
   g.inv_rows = 1.f / rows;
-  const cudaError_t e =
-      launch_forward<1, FEATURES, true>(g, static_cast<cudaStream_t>(cuda_stream));
+  cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
+  const cudaError_t e = cl == 2 ? launch_forward<1, FEATURES, true, 2>(g, s)
+                                : launch_forward<1, FEATURES, true, 1>(g, s);
   if (e != cudaSuccess) return cuda_fail(e, "pe_mlp_forward");
   count_launches(1);
   return PE_OK;
@@ -931,12 +1174,12 @@ int pe_mlp_backward(const pe_mlp_net *net, const void *feat, int rows, const flo
         (reinterpret_cast<uintptr_t>(z[l]) | reinterpret_cast<uintptr_t>(dz[l])) % 32 ||
         reinterpret_cast<uintptr_t>(gw[l]) % 16)
       return fail(PE_EINVAL, "mlp_backward: buffers of every layer required, aligned");
-    if (l > 0) map(&b.wt[l], net->w16t[l], H, H, H);
+    if (l > 0) map(&b.wt[l], net->w16t[l], H, H, H / BCL);
+    if (r == CUDA_SUCCESS) r = make_z_map(&b.zmap[l], z[l], rows);
     map(&w.dz[l], dz[l], rows, H, 64);
     map(&w.prev[l], l == 0 ? feat : h[l - 1], rows, K, 64);
-    b.z[l] = z[l];
     b.dz[l] = static_cast<__nv_bfloat16 *>(dz[l]);
-    b.gb[l] = gb[l];
+    w.gb[l] = gb[l];
     w.gw[l] = gw[l];
   }
   if (r != CUDA_SUCCESS) return fail(PE_EINVAL, "mlp_backward: tensor map encoding failed");
@@ -948,17 +1191,17 @@ int pe_mlp_backward(const pe_mlp_net *net, const void *feat, int rows, const flo
   w.width0 = net->in_width;
   w.ksteps = rows / 64;
   cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-  constexpr int bytes = BackwardLayout::BYTES + 1024;
-  cudaError_t e = cudaFuncSetAttribute(backward_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = cudaFuncSetAttribute(weight_grad_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, G_BYTES);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             G_BYTES);
+    e = launch_tiles(backward_kernel, rows / TM * BCL, BCL, BackwardLayout::BYTES + 1024, s, b);
   if (e != cudaSuccess) return cuda_fail(e, "pe_mlp_backward");
-  backward_kernel<<<rows / TM, THREADS, bytes, s>>>(b);
-  // about one CTA per SM, none with fewer than two 64-row steps
+  // about one CTA per SM, none with fewer than two 64-row steps; nor more than
+  // eight (chains of 16 MMAs into each accumulator: twice that at 16384 rows
+  // put the gradients 4.9e-7 from 64 bits, against 2.7e-7)
   const int tiles = 2 * net->layers;
-  const int splits = std::max(1, std::min(148 / tiles, w.ksteps / 2));
+  const int splits =
+      std::max({1, std::min(148 / tiles, w.ksteps / 2), (w.ksteps + 7) / 8});
   weight_grad_kernel<<<dim3(tiles, splits), G_THREADS, G_BYTES, s>>>(w);
   PE_CUDA_TRY(cudaGetLastError());
   count_launches(2);

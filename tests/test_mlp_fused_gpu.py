@@ -133,3 +133,33 @@ def test_silu_at_extreme_pre_activations():
         else:
             assert torch.equal(torch.isnan(h), torch.full_like(h, float(want)).isnan())
             assert not torch.isfinite(h).any()
+
+
+@pytest.mark.parametrize("layers", [1, 2, 4])
+def test_two_ctas_per_tile_equal_one(layers):
+    """A forward training pass shares a 128-row tile between two CTAs up to 74
+    tiles (9472 rows) and gives it to one from 75: the same rows either way, and
+    their backward pass."""
+    many, few = 9600, 9472
+    net = make_net(layers, many)
+    runs = []
+    for rows in (many, few):
+        net.loss.zero_()
+        net.forward(rows, target=True)
+        # the mean's 1 / rows is the one difference between the two calls
+        net.dy.copy_((net.y - net.target) * (2.0 / many))
+        net.backward(rows)
+        torch.cuda.synchronize()
+        runs.append([t[:few].clone() for t in [net.y] + net.z + net.h + net.dz])
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
+    # FP32 sums of the second run: at most 608 roundings of 2^-24 (chains of 16
+    # rows, 8 ranges and 74 tiles) on the sum of magnitudes
+    bound = 608 * 2.0 ** -24
+    pairs = [(net.grads[layers + l], net.dz[l][:few].double()) for l in range(layers)]
+    dy = net.dy[:few].double()[:, None]
+    pairs.append((net.grads[2 * layers], dy * net.h[-1][:few].double()))
+    pairs.append((net.grads[2 * layers + 1], dy))
+    for got, terms in pairs:
+        err = (got.double().flatten() - terms.sum(0)).abs()
+        assert bool((err <= bound * terms.abs().sum(0) + 1e-30).all())
