@@ -1,15 +1,17 @@
 """Tile autotuner of the batched solver.
 
-A work item of the exact batched kernel is `rows` y rows of one (vP, vE,
-psi) plane of one solve; one of the tiled float32 kernel is `rows` y rows of
-one (vP, vE) plane stack over all headings, a thread per 4-cell x chunk (at
-most 256 / ceil(positions / 4) rows).  Fewer rows give more, smaller items
+A work item of the tiled kernels is `rows` y rows of one (vP, vE) plane stack
+of one solve over all headings (float32) or a chunk of them that the solver
+picks (exact), a thread per 4-cell x chunk (at most 256 / ceil(positions / 4)
+rows; larger tables are held to that).  Fewer rows give more, smaller items
 (better balance across the CTAs); more rows the reverse (less y halo per
 cell), and the best choice depends on the grid width.  `tune` times every candidate row count on a few
 solves of each width bucket (each solve cut to a short horizon, so a trial
 is a few RK2 steps) and keeps the fastest; the winners are cached in a JSON
 file keyed by device name and arithmetic, and `apply` sets them on a
-`BatchSolver`.
+`BatchSolver`.  An exact solve's default, its rows spread evenly over the
+fewest slabs, is timed too and recorded as 0 where it wins (positions 18 to
+39: 22.5 ms, 25.6 to 73 ms with one row count for all).
 """
 
 from __future__ import annotations
@@ -46,9 +48,9 @@ def _device_name(device):
 
 def candidates(narrowest, local_precision="float64", widest=None):
     """Row counts to try for a bucket whose grids have `narrowest` to
-    `widest` positions: exact kernel, those that give every thread of a
-    256-thread CTA a cell; tiled float32 kernel, those up to the capacity of
-    a CTA on the widest grid (one 4-cell chunk per thread)."""
+    `widest` positions: exact solves, those of at least 256 cells (beside the
+    default); float32, those up to the capacity of a CTA on the widest grid
+    (one 4-cell chunk per thread)."""
     if local_precision == "float32":
         widest = narrowest if widest is None else max(widest, narrowest)
         cap = min(narrowest, 256 // ((widest + 3) // 4))
@@ -59,12 +61,13 @@ def candidates(narrowest, local_precision="float64", widest=None):
 
 def tune(solves, *, device=0, local_precision="float32", per_bucket=6, trial_steps=4,
          repeats=2, cache=None, log=None):
-    """Fastest rows per width bucket for these solves: {bucket: rows}."""
+    """Fastest rows per width bucket for these solves: {bucket: rows}, 0 for
+    each solve's default."""
     import torch
 
     cache = Path(cache) if cache else default_cache()
-    key = f"{_device_name(device)} {local_precision}" + (" tiled" if local_precision == "float32"
-                                                         else "")
+    # (tables without "tiled" hold the rows of kernels of a cell per thread)
+    key = f"{_device_name(device)} {local_precision} tiled"
     try:
         table = json.loads(cache.read_text())
     except (OSError, ValueError):
@@ -85,9 +88,11 @@ def tune(solves, *, device=0, local_precision="float32", per_bucket=6, trial_ste
         trial = [replace(s, horizon=trial_steps * lim) for s, lim in zip(sample, limits)]
         with BatchSolver(trial, local_precision=local_precision, device=device) as b:
             widths = [s.grid.positions for s in members]
-            for rows in candidates(min(widths), local_precision, max(widths)):
+            default = [0] if local_precision == "float64" else []
+            for rows in default + candidates(min(widths), local_precision, max(widths)):
                 for i in range(len(trial)):
-                    b.set_tile(i, rows)
+                    if rows:
+                        b.set_tile(i, rows)
                 best = None
                 for _ in range(repeats):
                     b.initialize()

@@ -15,7 +15,7 @@ from tests.helpers import A3
 pytestmark = pytest.mark.gpu
 
 GRIDS = [RelativeGrid(19, 12, 15, 13, 4.0), RelativeGrid(21, 8, 17, 16, 4.0),
-         RelativeGrid(22, 13, 14, 12, 6.0), RelativeGrid(36, 9, 9, 9, 6.0),
+         RelativeGrid(22, 13, 16, 14, 6.0), RelativeGrid(36, 9, 9, 9, 6.0),
          RelativeGrid(65, 13, 5, 6, 8.0)]
 
 
@@ -104,3 +104,22 @@ def test_tiled_batch_of_one_equals_the_single_grid(positions, headings, rows):
             np.testing.assert_array_equal(field.view(np.uint32), s.field().view(np.uint32))
             np.testing.assert_array_equal(arrival.view(np.uint32), s.arrival().view(np.uint32))
             assert stats == s.stats()
+
+
+def test_exact_autotune_may_keep_the_default_tile(tmp_path):
+    from dataclasses import replace
+
+    from pursuit_evasion_b200.batch import BatchSolver, autotune, draw_batch
+
+    solves = [replace(s, horizon=0.05) for s in draw_batch(4, count=2)]
+    cache = tmp_path / "tiles.json"
+    table = autotune.tune(solves, local_precision="float64", trial_steps=1, cache=cache)
+    for bucket, rows in table.items():
+        widths = [s.grid.positions for s in solves
+                  if autotune.bucket_of(s.grid.positions) == bucket]
+        assert rows in [0] + autotune.candidates(min(widths), "float64", max(widths))
+    assert autotune.tune(solves, local_precision="float64", cache=cache) == table
+    with BatchSolver(solves, local_precision="float64") as b:
+        before = [b.tile(i) for i in range(len(solves))]
+        autotune.apply(b, {bucket: 0 for bucket in table})
+        assert [b.tile(i) for i in range(len(solves))] == before
