@@ -23,7 +23,7 @@
 struct pe_relative_shard {
   pe_relative_params p{};
   pe::Rel5Grid g{};  // global geometry; own_lo / own_n / slab_lo set
-  pe::Rel5Tile tile{};  // float32 stage tiling
+  pe::Rel5Tile tile{};  // stage tiling
   int lo = 0, hi = 0, own_lo = 0, own_hi = 0;
   double t = 0;
   int64_t steps = 0;

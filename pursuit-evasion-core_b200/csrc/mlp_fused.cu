@@ -1089,8 +1089,8 @@ cudaError_t launch_forward(ForwardArgs &g, cudaStream_t stream) {
 }
 
 // CTAs per 128-row tile of a forward training pass: two while that many fit the
-// SMs (8192 rows 43.6 us with one, 34.6 with two), one beyond (9600 rows 41.4
-// with one, 64.1 with two, which then take a second wave; 65536: 167 and 240).
+// SMs (8192 rows 43.6 us with one, 34.6 with two), one beyond (9600 rows 40.4
+// with one, 64.1 with two, which then take a second wave; 65536: 163 and 240).
 // The backward pass takes two at every size (9600 rows, with the weight
 // gradients, 74 us with one, 72 with two; 19072: 144, 111; 65536: 325, 278).
 inline int cluster_of(int rows) { return 2 * (rows / TM) <= 148 ? 2 : 1; }

@@ -4,6 +4,9 @@
 // -fmad=false: no multiply-add contraction, IEEE double division, so each
 // stored float equals the reference CPU's bit for bit.
 //
+// The kernel of grids under about 0.6 M cells and of layouts without padding;
+// larger ones take tiles (relative5d_tiled_exact.cu).
+//
 // One thread per cell of the padded layout.  blockIdx.y enumerates (vP, vE),
 // blockIdx.z the heading, and the x dimension covers the (y, x) plane, so
 // that the CTAs in flight cover the speed neighbours of one heading (their
