@@ -24,6 +24,7 @@ struct pe_batch {
   int device = 0;
   bool exact = true;
   bool tiled = true;  // the tiled kernels; else (exact) a cell per thread
+  bool wide = false;  // rows of several parts (rel5_batch_row_parts)
   std::vector<pe_relative_params> params;  // caller's order
   std::vector<double> horizons;
   std::vector<pe::Rel5Grid> grids;
@@ -146,10 +147,10 @@ int upload_descriptors(pe_batch *h) {
       s.items = (int64_t)g.nvp * g.nve * g.nh * ((g.nx + s.rows - 1) / s.rows);
     } else {
       // item: `rows` y rows of one (vP, vE) plane stack, all headings
-      // (float32) or a chunk of them (exact)
+      // (float32, a part of a row where it is wide) or a chunk of them (exact)
       s.rows = pe::rel5_batch_tiled_rows(g.nx, g.xp, h->rows[i]);
       s.items = (int64_t)g.nvp * g.nve * ((g.nx + s.rows - 1) / s.rows) *
-                (h->exact ? (g.nh + s.chunk - 1) / s.chunk : 1);
+                (h->exact ? (g.nh + s.chunk - 1) / s.chunk : pe::rel5_batch_row_parts(g.xp));
       smem = std::max(smem, pe::rel5_batch_tiled_smem(s.rows, g.xp));
     }
     s.item_base = base;
@@ -159,7 +160,8 @@ int upload_descriptors(pe_batch *h) {
     // a different launch shape: size the cooperative grid again and record
     // a new graph at the next run
     h->tiled_smem = smem;
-    h->grid = h->exact ? pe::rel5_batch_grid_tiled_exact(smem) : pe::rel5_batch_grid_tiled(smem);
+    h->grid = h->exact ? pe::rel5_batch_grid_tiled_exact(smem)
+                       : pe::rel5_batch_grid_tiled(smem, h->wide);
     if (h->grid <= 0) return fail(PE_EINVAL, "batch tiles do not fit the tiled kernel");
     if (h->graph) {
       cudaGraphExecDestroy(h->graph);
@@ -201,7 +203,7 @@ int capture(pe_batch *h) {
     err = !h->tiled ? pe::rel5_batch_run_exact(args, h->grid, h->stream)
           : h->exact
               ? pe::rel5_batch_run_tiled_exact(args, h->grid, h->tiled_smem, h->stream)
-              : pe::rel5_batch_run_tiled(args, h->grid, h->tiled_smem, h->stream);
+              : pe::rel5_batch_run_tiled(args, h->grid, h->tiled_smem, h->wide, h->stream);
   cudaError_t end = cudaStreamEndCapture(h->stream, &g);
   if (err == cudaSuccess) err = end;
   if (err == cudaSuccess) err = cudaGraphInstantiate(&h->graph, g, 0);
@@ -274,8 +276,7 @@ int pe_batch_create(const pe_relative_params *params, const double *horizons, in
     const int widest = pe::rel5_batch_tiled_rows(g.nx, g.xp, 0);
     const int slabs = (g.nx + widest - 1) / widest;
     h->rows.push_back(h->exact ? (g.nx + slabs - 1) / slabs : widest);
-    // rows wider than a CTA's threads take a cell per thread
-    if (h->exact && g.xp / 4 > pe::kRel5BatchThreads) h->tiled = false;
+    if (pe::rel5_batch_row_parts(g.xp) > 1) h->wide = true;
     h->field_off.push_back(fields);
     fields += 3 * (size_t)g.n_padded;
     h->table_off.push_back(tables);
@@ -285,6 +286,8 @@ int pe_batch_create(const pe_relative_params *params, const double *horizons, in
     h->plane_off.push_back(planes);
     planes += (size_t)g.nx * g.nx;
   }
+  // exact rows wider than a CTA's threads take a cell per thread
+  h->tiled = !(h->exact && h->wide);
   h->order.resize(count);
   std::iota(h->order.begin(), h->order.end(), 0);
   std::stable_sort(h->order.begin(), h->order.end(), [&](int x, int y) {

@@ -51,15 +51,22 @@ int rel5_batch_grid_tiled_exact(size_t smem);
 cudaError_t rel5_batch_run_tiled_exact(const Rel5BatchArgs &args, int grid, size_t smem,
                                        cudaStream_t stream);
 
+// Parts of a row that a CTA takes as items of their own: a row of more 4-cell
+// chunks than threads (over 1,024 positions) is split, others are one part.
+__host__ __device__ inline int rel5_batch_row_parts(int xp) {
+  return (xp / 4 + kRel5BatchThreads - 1) / kRel5BatchThreads;
+}
+
 // Float32 update, tiled (relative5d_batch_tiled.cu): a work item is `rows` y
-// rows of one (vP, vE) plane stack, all headings, one thread per 4-cell x
-// chunk.  rows: the tile clamped to the CTA (want < 1: the largest that
+// rows (or a part of one) of one (vP, vE) plane stack, all headings, one thread
+// per 4-cell x chunk.  rows: the tile clamped to the CTA (want < 1: the largest that
 // fits); smem: dynamic shared memory of a CTA for that tile; grid: CTAs of
-// one cooperative launch with that shared memory.
+// one cooperative launch with that shared memory; wide: some rows have several
+// parts.
 int rel5_batch_tiled_rows(int nx, int xp, int want);
 size_t rel5_batch_tiled_smem(int rows, int xp);
-int rel5_batch_grid_tiled(size_t smem);
-cudaError_t rel5_batch_run_tiled(const Rel5BatchArgs &args, int grid, size_t smem,
+int rel5_batch_grid_tiled(size_t smem, bool wide);
+cudaError_t rel5_batch_run_tiled(const Rel5BatchArgs &args, int grid, size_t smem, bool wide,
                                  cudaStream_t stream);
 
 }  // namespace pe

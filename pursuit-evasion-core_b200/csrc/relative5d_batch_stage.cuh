@@ -41,8 +41,10 @@ __host__ __device__ inline int buffer_floats(int rows, int xp) {
   return (rows + 4) * xp + kNb * rows * xp;
 }
 
+// A thread of an item owns chunk c0 + (thread mod xc) of one of its rows.
 struct ItemGeom {
   int iv, ie, y0, r_eff, R, xc;
+  int c0 = 0;
 };
 
 // Stage heading `psi` of an item into buffer `buf` (called by warp 0): the

@@ -4,17 +4,18 @@
 // the arithmetic of the single-grid float32 kernel (relative5d_fast.cu).
 //
 // A work item is `rows` y rows of one (vP, vE) plane stack of one solve, all
-// headings.  A thread owns a 4-cell x chunk of one row and walks the
-// headings, carrying the heading differences and ENO selections from one
-// heading to the next (the psi stencil).  For each heading the CTA stages,
-// double-buffered against the previous heading's arithmetic, the item's own
-// plane rows with a 2-row y halo and the rows of the 8 speed-neighbour
-// planes (vE +-1, +-2, vP +-1, +-2): lanes 0-8 of warp 0 issue one bulk
-// copy (cp.async.bulk, the TMA engine) each, one per contiguous row range,
-// all completing on the buffer's mbarrier, on which every thread waits
-// (bounded); the x, y and speed stencils then read shared
-// memory.  The persistent loop over steps, the active-item prefix and the
-// bounded grid barrier are those of relative5d_batch_impl.cuh.
+// headings; of a row with more 4-cell chunks than the CTA has threads (over
+// 1,024 positions) it is a part of that many chunks.  A thread owns a 4-cell x
+// chunk of one row and walks the headings, carrying the heading differences
+// and ENO selections from one heading to the next (the psi stencil).  For each
+// heading the CTA stages, double-buffered against the previous heading's
+// arithmetic, the item's own plane rows with a 2-row y halo and the rows of
+// the 8 speed-neighbour planes (vE +-1, +-2, vP +-1, +-2): lanes 0-8 of warp 0
+// issue one bulk copy (cp.async.bulk, the TMA engine) each, one per contiguous
+// row range, all completing on the buffer's mbarrier, on which every thread
+// waits (bounded); the x, y and speed stencils then read shared memory.  The
+// persistent loop over steps, the active-item prefix and the bounded grid
+// barrier are those of relative5d_batch_impl.cuh.
 #include "relative5d_batch_stage.cuh"
 #include "relative5d_eno_f32.cuh"
 
@@ -23,9 +24,9 @@ namespace {
 
 using namespace eno32;
 
-// One stage of one item (all headings).  Returns the largest |change| of
+// One stage of one item (all headings; WIDE: of a part of a row).  Returns the largest |change| of
 // this thread's cells (stage 2) and flags non-finite values.
-template <int ORDER, int BLEND>
+template <int ORDER, int BLEND, bool WIDE>
 __device__ __forceinline__ void item_stage(const Rel5Grid &g, const Rel5Stage &s,
                                            const ItemGeom &it, float *smem, StageRing &ring,
                                            float &change_max, float &change_up,
@@ -33,9 +34,9 @@ __device__ __forceinline__ void item_stage(const Rel5Grid &g, const Rel5Stage &s
   const int xp = g.xp, xc = it.xc;
   const int64_t PP = (int64_t)g.nx * xp;
   const int tid = threadIdx.x;
-  const int r = tid / xc, c = tid - (tid / xc) * xc;
-  const bool active = tid < it.R * xc && r < it.r_eff;
-  const int x0 = 4 * c, iy = it.y0 + r;
+  const int r = tid / xc, x0 = 4 * ((WIDE ? it.c0 : 0) + tid - r * xc);
+  const bool active = tid < it.R * xc && r < it.r_eff && (!WIDE || x0 < xp);
+  const int iy = it.y0 + r;
   const int bufsz = buffer_floats(it.R, xp);
 
   const float ext = (float)g.extent, dxf = (float)g.dx;
@@ -304,13 +305,14 @@ __device__ __forceinline__ void item_stage(const Rel5Grid &g, const Rel5Stage &s
   __syncthreads();  // the buffers are restaged by the next item
 }
 
-template <int BLEND>
-__device__ __forceinline__ void tiled_stage(const Rel5BatchArgs &A, int step, int64_t n_items, double *scratch,
-                            Rel5Grid *sg, float *smem, StageRing &ring) {
+template <int BLEND, bool WIDE>
+__device__ __forceinline__ void tiled_stage(const Rel5BatchArgs &A, int step, int64_t n_items,
+                                            double *scratch, Rel5Grid *sg, float *smem,
+                                            StageRing &ring) {
   int64_t lo = 0, hi = 0;
   const Rel5BatchSolve *S = nullptr;
   Rel5Stage s{};
-  int rows = 1, slabs = 1, xc = 1;
+  int rows = 1, slabs = 1, xc = 1, parts = 1;
   float change_max = 0.f, change_up = 0.f;
   float2 finite_acc = make_float2(0.f, 0.f);
   auto flush = [&]() {
@@ -349,10 +351,18 @@ __device__ __forceinline__ void tiled_stage(const Rel5BatchArgs &A, int step, in
       __syncthreads();
       slabs = (sg->nx + rows - 1) / rows;
       xc = sg->xp / 4;
+      if (WIDE) {
+        parts = rel5_batch_row_parts(sg->xp);
+        if (parts > 1) xc = kThreads;
+      }
     }
     const Rel5Grid &g = *sg;
     int64_t local = item - lo;
     ItemGeom it;
+    if (WIDE) {
+      it.c0 = (int)(local % parts) * kThreads;
+      local /= parts;
+    }
     const int slab = (int)(local % slabs);
     local /= slabs;
     it.ie = (int)(local % g.nve);
@@ -361,11 +371,15 @@ __device__ __forceinline__ void tiled_stage(const Rel5BatchArgs &A, int step, in
     it.xc = xc;
     it.y0 = slab * rows;
     it.r_eff = min(rows, g.nx - it.y0);
-    item_stage<2, BLEND>(g, s, it, smem, ring, change_max, change_up, finite_acc);
+    item_stage<2, BLEND, WIDE>(g, s, it, smem, ring, change_max, change_up, finite_acc);
   }
   flush();
 }
 
+// WIDE: some rows have more chunks than the CTA has threads.  A kernel of its
+// own: with the row parts in the one for all sizes, 64 solves of 17-49 positions
+// took 125.1 against 124.4 ms.
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads, 2)
     rel5_batch_tiled_kernel(const Rel5BatchArgs A) {
   extern __shared__ __align__(16) float smem[];
@@ -387,12 +401,12 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < A.count;
          k += gridDim.x * blockDim.x)
       if (step < A.solves[k].nsteps) A.solves[k].stats->residual = 0ull;
-    tiled_stage<0>(A, step, n_items, scratch, &sg, smem, ring);
+    tiled_stage<0, WIDE>(A, step, n_items, scratch, &sg, smem, ring);
     if (!batch_impl::grid_barrier(A.sync, ++round)) break;
     // the next stage's bulk copies read what other CTAs stored before the
     // barrier: order it for the async proxy (warp 0 issues the copies)
     if (threadIdx.x < 32) bulk::fence_async_global();
-    tiled_stage<1>(A, step, n_items, scratch, &sg, smem, ring);
+    tiled_stage<1, WIDE>(A, step, n_items, scratch, &sg, smem, ring);
     if (!batch_impl::grid_barrier(A.sync, ++round)) break;
     if (threadIdx.x < 32) bulk::fence_async_global();
   }
@@ -418,21 +432,22 @@ size_t rel5_batch_tiled_smem(int rows, int xp) {
   return 2 * sizeof(float) * (size_t)buffer_floats(rows, xp);
 }
 
-int rel5_batch_grid_tiled(size_t smem) {
+int rel5_batch_grid_tiled(size_t smem, bool wide) {
+  auto kernel = wide ? rel5_batch_tiled_kernel<true> : rel5_batch_tiled_kernel<false>;
   int device = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&device) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
     return 0;
-  if (cudaFuncSetAttribute(rel5_batch_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
     return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rel5_batch_tiled_kernel, kThreads,
-                                                    smem) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) !=
+      cudaSuccess)
     return 0;
   return sms * per_sm;
 }
 
-cudaError_t rel5_batch_run_tiled(const Rel5BatchArgs &args, int grid, size_t smem,
+cudaError_t rel5_batch_run_tiled(const Rel5BatchArgs &args, int grid, size_t smem, bool wide,
                                  cudaStream_t stream) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
@@ -444,7 +459,8 @@ cudaError_t rel5_batch_run_tiled(const Rel5BatchArgs &args, int grid, size_t sme
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, rel5_batch_tiled_kernel, args);
+  return wide ? cudaLaunchKernelEx(&cfg, rel5_batch_tiled_kernel<true>, args)
+              : cudaLaunchKernelEx(&cfg, rel5_batch_tiled_kernel<false>, args);
 }
 
 }  // namespace pe

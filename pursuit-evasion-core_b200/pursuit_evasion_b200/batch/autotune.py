@@ -53,7 +53,7 @@ def candidates(narrowest, local_precision="float64", widest=None):
     (one 4-cell chunk per thread)."""
     if local_precision == "float32":
         widest = narrowest if widest is None else max(widest, narrowest)
-        cap = min(narrowest, 256 // ((widest + 3) // 4))
+        cap = max(1, min(narrowest, 256 // ((widest + 3) // 4)))
         return sorted({min(r, cap) for r in CANDIDATE_ROWS if r <= narrowest} | {cap})
     rows = [r for r in CANDIDATE_ROWS if r <= narrowest and r * narrowest >= 256]
     return rows or [narrowest]

@@ -47,6 +47,12 @@ def test_buckets_and_candidates():
     assert max(autotune.candidates(34, "float32", 40)) * 10 <= 256
 
 
+def test_float32_candidates_of_rows_wider_than_a_cta():
+    # (over 1,024 positions a row is split over items: one row each)
+    assert autotune.candidates(1025, "float32") == [1]
+    assert autotune.candidates(40, "float32", 1300) == [1]
+
+
 @pytest.mark.parametrize("field, value", [("order", 1), ("precision", _native.PE_LOCAL_F32),
                                           ("positions", 2)])
 def test_create_rejects_unsupported_options(field, value):
