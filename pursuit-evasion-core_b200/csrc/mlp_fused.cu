@@ -46,6 +46,7 @@
 #include "mlp_tc.cuh"
 
 #include <algorithm>
+#include <cfloat>
 
 namespace pe {
 namespace {
@@ -240,12 +241,13 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 }
 __device__ __forceinline__ float2 two(float a) { return make_float2(a, a); }
 
-// -(1 + exp(-z)) of a pair, not below -2^125 (its reciprocal stays normal;
-// SiLU is below 3e-36 there).
+// -(1 + exp(-z)) of a pair, finite.  Its approximate reciprocal is 0 beyond
+// 2^126 (z < -87.34, where SiLU is above -1.03e-36), and with it SiLU and its
+// derivative, however large -z is.
 __device__ __forceinline__ float2 neg_denominator(float2 z) {
   const float2 x = __fmul2_rn(z, two(-1.44269504f));
   const float2 nd = __ffma2_rn(make_float2(ex2(x.x), ex2(x.y)), two(-1.f), two(-1.f));
-  return make_float2(max_nan(nd.x, -0x1p125f), max_nan(nd.y, -0x1p125f));
+  return make_float2(max_nan(nd.x, -FLT_MAX), max_nan(nd.y, -FLT_MAX));
 }
 // 1 / -nd by the approximate reciprocal and one Newton step
 __device__ __forceinline__ float2 reciprocal(float2 nd) {
