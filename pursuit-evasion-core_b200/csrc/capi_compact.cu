@@ -24,6 +24,7 @@
 #include <utility>
 #include <vector>
 
+#include "launch_shape.cuh"
 #include "pe_internal.h"
 
 namespace pe {
@@ -639,8 +640,7 @@ int configure_launch(pe_compact *h, int rcap) {
   if (h->d.npa <= pe::kMaxActions && h->d.ne <= 65536 && group >= 2) {
     const void *kernel = h->packed ? (const void *)pe::backup_all_kernel<true>
                                    : (const void *)pe::backup_all_kernel<false>;
-    PE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)all_smem));
+    PE_CUDA_TRY(pe::allow_all_smem(kernel));
     int resident = 0;
     PE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, pe::kThreads,
                                                               all_smem));
@@ -662,8 +662,7 @@ int configure_launch(pe_compact *h, int rcap) {
                                : (const void *)pe::backup_kernel<true, false>)
                 : (h->smem_row ? (const void *)pe::backup_kernel<false, true>
                                : (const void *)pe::backup_kernel<false, false>);
-  PE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)h->smem));
+  PE_CUDA_TRY(pe::allow_all_smem(kernel));
   int resident = 0;
   PE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, pe::kThreads,
                                                             h->smem));

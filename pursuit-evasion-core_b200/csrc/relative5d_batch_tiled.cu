@@ -16,6 +16,7 @@
 // waits (bounded); the x, y and speed stencils then read shared memory.  The
 // persistent loop over steps, the active-item prefix and the bounded grid
 // barrier are those of relative5d_batch_impl.cuh.
+#include "launch_shape.cuh"
 #include "relative5d_batch_stage.cuh"
 #include "relative5d_eno_f32.cuh"
 
@@ -434,17 +435,7 @@ size_t rel5_batch_tiled_smem(int rows, int xp) {
 
 int rel5_batch_grid_tiled(size_t smem, bool wide) {
   auto kernel = wide ? rel5_batch_tiled_kernel<true> : rel5_batch_tiled_kernel<false>;
-  int device = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&device) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-    return 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) !=
-      cudaSuccess)
-    return 0;
-  return sms * per_sm;
+  return cooperative_ctas(reinterpret_cast<const void *>(kernel), kThreads, smem);
 }
 
 cudaError_t rel5_batch_run_tiled(const Rel5BatchArgs &args, int grid, size_t smem, bool wide,

@@ -15,6 +15,7 @@
 // positions, 6.7e8 cell-stages: 56 ms on the cell-per-thread kernel, 22.7 ms
 // here; 32 solves, 7.7e9: 233 ms.  Handling two of the four cells at a time
 // keeps fewer values live but measured 22 % slower.
+#include "launch_shape.cuh"
 #include "relative5d_batch_stage.cuh"
 #include "relative5d_exact_walk.cuh"
 
@@ -207,18 +208,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 }  // namespace
 
 int rel5_batch_grid_tiled_exact(size_t smem) {
-  int device = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&device) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-    return 0;
-  if (cudaFuncSetAttribute(rel5_batch_tiled_exact_kernel,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rel5_batch_tiled_exact_kernel,
-                                                    kThreads, smem) != cudaSuccess)
-    return 0;
-  return sms * per_sm;
+  return cooperative_ctas(reinterpret_cast<const void *>(rel5_batch_tiled_exact_kernel), kThreads,
+                          smem);
 }
 
 cudaError_t rel5_batch_run_tiled_exact(const Rel5BatchArgs &args, int grid, size_t smem,

@@ -41,6 +41,7 @@
 #include <algorithm>
 #include <cstdio>
 
+#include "launch_shape.cuh"
 #include "relative5d.cuh"
 #include "relative5d_eno_f32.cuh"
 #include "relative5d_ring.cuh"
@@ -450,29 +451,14 @@ int g_last_resident = 0;
 
 template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0, bool OVERLAP = false>
 cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
-  // Resident CTAs per SM for this (shared memory, block size); recomputed
-  // when either changes.
-  static int configured_smem = 0, configured_threads = 0;
-  static int resident = 0;
-  if (configured_smem != (int)smem || configured_threads != threads || resident == 0) {
-    cudaError_t e = cudaFuncSetAttribute(rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &resident, rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>, threads, smem);
-    if (e != cudaSuccess) return e;
-    if (resident < 1) return cudaErrorInvalidConfiguration;
-    configured_smem = (int)smem;
-    configured_threads = threads;
-  }
-  int device = 0, sms = 0;
-  cudaGetDevice(&device);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const int blocks = std::min(args.items, sms * resident);
-  g_last_resident = resident;
-  return launch_overlapped(OVERLAP, rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>,
-                           dim3((unsigned)blocks), threads, smem, stream, args);
+  auto kernel = rel5_stage_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>;
+  static thread_local LaunchShape shape;
+  const cudaError_t e =
+      launch_shape(reinterpret_cast<const void *>(kernel), threads, smem, shape);
+  if (e != cudaSuccess) return e;
+  const int blocks = std::min(args.items, shape.sms * shape.resident);
+  g_last_resident = shape.resident;
+  return launch_overlapped(OVERLAP, kernel, dim3((unsigned)blocks), threads, smem, stream, args);
 }
 
 template <int ORDER, int BLEND, bool OVERLAP>

@@ -13,6 +13,7 @@
 // (relative5d_exact_walk.cuh): about 165 double operations per cell, which
 // bound it (64 per clock and SM): 1.77 ms per stage at 65x48x21x21 (4.0 ms
 // for the thread-per-cell kernel), of which the double operations are 0.85.
+#include "launch_shape.cuh"
 #include "relative5d_exact_walk.cuh"
 #include "relative5d_ring.cuh"
 
@@ -156,28 +157,13 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
 template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0, bool OVERLAP = false>
 cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
   auto kernel = rel5_walk_exact_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>;
-  // co-resident CTAs of the last (device, shared memory, block size) this
-  // thread launched
-  struct Shape {
-    int device = -1, smem = 0, threads = 0, ctas = 0;
-  };
-  static thread_local Shape last;
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
+  static thread_local LaunchShape shape;
+  const cudaError_t e =
+      launch_shape(reinterpret_cast<const void *>(kernel), threads, smem, shape);
   if (e != cudaSuccess) return e;
-  if (last.device != device || last.smem != (int)smem || last.threads != threads) {
-    int sms = 0, resident = 0;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, threads, smem);
-    if (e != cudaSuccess) return e;
-    if (resident < 1) return cudaErrorInvalidConfiguration;
-    last = Shape{device, (int)smem, threads, sms * resident};
-  }
   return launch_overlapped(OVERLAP, kernel,
-                           dim3((unsigned)std::min(args.items, last.ctas)), threads, smem,
+                           dim3((unsigned)std::min(args.items, shape.sms * shape.resident)), threads,
+                           smem,
                            stream, args);
 }
 

@@ -35,6 +35,7 @@
 // Preconditions (checked on the host): nx + 4 <= 72, every successor within
 // 1.99 cells of its cell in x and y, heading shifts below one plane, and
 // speed successors inside the three staged slabs.
+#include "launch_shape.cuh"
 #include "semilag5d.cuh"
 
 namespace pe {
@@ -500,20 +501,11 @@ template <int MODE>
 cudaError_t launch(const SLGrid &g, const SLBackup &b, const SLTiled &t,
                    const SLTiledPlan &plan, cudaStream_t stream) {
   auto kernel = sl_tiled_kernel<MODE, kCPT>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)plan.smem);
+  static thread_local LaunchShape shape;
+  const cudaError_t err =
+      launch_shape(reinterpret_cast<const void *>(kernel), plan.threads, plan.smem, shape);
   if (err != cudaSuccess) return err;
-  int device = 0, sms = 0;
-  err = cudaGetDevice(&device);
-  if (err != cudaSuccess) return err;
-  err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (err != cudaSuccess) return err;
-  int resident = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, plan.threads,
-                                                      plan.smem);
-  if (err != cudaSuccess) return err;
-  const int64_t slots = (int64_t)sms * (resident > 0 ? resident : 1);
+  const int64_t slots = (int64_t)shape.sms * shape.resident;
   const int64_t grid = plan.items < slots ? plan.items : slots;
   kernel<<<(unsigned)grid, plan.threads, plan.smem, stream>>>(g, b, t, plan);
   return cudaGetLastError();

@@ -31,6 +31,7 @@
 // 2.79 -> 1.12 ms; it is the faster one down to the smallest grid (5x4x3x3: 35
 // -> 31 us).  The x and y axes of a cell share their spacing and go through
 // packed FP32 together (7 % of the step).
+#include "launch_shape.cuh"
 #include "world8d_column.cuh"
 #include "world8d_stage.cuh"
 
@@ -536,28 +537,11 @@ int group_columns(const World8Grid &g) {
 template <int ORDER, int NE, int SKIND>
 cudaError_t launch_kind(const ColExactArgs &a, size_t smem, cudaStream_t stream) {
   auto kernel = world8_column_exact_kernel<ORDER, NE, SKIND>;
-  struct Shape {
-    int device = -1, ctas = 0;
-    size_t smem = 0;
-  };
-  static thread_local Shape last;
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
+  static thread_local LaunchShape shape;
+  const cudaError_t e = launch_shape(reinterpret_cast<const void *>(kernel), kT, smem, shape);
   if (e != cudaSuccess) return e;
-  if (last.device != device || last.smem != smem) {
-    int sms = 0, resident = 0;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kT, smem);
-    if (e != cudaSuccess) return e;
-    if (resident < 1) return cudaErrorInvalidConfiguration;
-    last.device = device;
-    last.smem = smem;
-    last.ctas = sms * resident;
-  }
-  kernel<<<a.outer < last.ctas ? a.outer : last.ctas, kT, smem, stream>>>(a);
+  const int ctas = shape.sms * shape.resident;
+  kernel<<<a.outer < ctas ? a.outer : ctas, kT, smem, stream>>>(a);
   return cudaGetLastError();
 }
 

@@ -21,6 +21,7 @@
 // of world8d_stage.cuh.
 #include <cstdio>
 
+#include "launch_shape.cuh"
 #include "relative5d_eno_f32.cuh"
 #include "world8d_column.cuh"
 #include "world8d_stage.cuh"
@@ -315,23 +316,11 @@ __global__ void __launch_bounds__(kThreads)
 
 template <int ORDER>
 cudaError_t launch_block(const FastW8Args &a, size_t smem, cudaStream_t stream) {
-  static size_t configured = 0;
-  static int resident = 0;
-  if (configured != smem || resident == 0) {
-    cudaError_t e = cudaFuncSetAttribute(world8_block_kernel<ORDER>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, world8_block_kernel<ORDER>,
-                                                      kThreads, smem);
-    if (e != cudaSuccess) return e;
-    if (resident < 1) return cudaErrorInvalidConfiguration;
-    configured = smem;
-  }
-  int device = 0, sms = 0;
-  cudaGetDevice(&device);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const int blocks = a.outer < sms * resident ? a.outer : sms * resident;
+  static thread_local LaunchShape shape;
+  const cudaError_t e = launch_shape(reinterpret_cast<const void *>(world8_block_kernel<ORDER>),
+                                     kThreads, smem, shape);
+  if (e != cudaSuccess) return e;
+  const int ctas = shape.sms * shape.resident, blocks = a.outer < ctas ? a.outer : ctas;
   world8_block_kernel<ORDER><<<blocks, kThreads, smem, stream>>>(a);
   return cudaGetLastError();
 }
@@ -673,21 +662,11 @@ __global__ void __launch_bounds__(kColThreads, 2)
 template <int ORDER, int NE, int SKIND>
 cudaError_t launch_column_kind(const ColW8Args &a, size_t smem, cudaStream_t stream) {
   auto kernel = world8_column_kernel<ORDER, NE, SKIND>;
-  static size_t configured = 0;
-  static int resident = 0;
-  if (configured != smem || resident == 0) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kColThreads, smem);
-    if (e != cudaSuccess) return e;
-    if (resident < 1) return cudaErrorInvalidConfiguration;
-    configured = smem;
-  }
-  int device = 0, sms = 0;
-  cudaGetDevice(&device);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  const int blocks = a.outer < sms * resident ? a.outer : sms * resident;
+  static thread_local LaunchShape shape;
+  const cudaError_t e =
+      launch_shape(reinterpret_cast<const void *>(kernel), kColThreads, smem, shape);
+  if (e != cudaSuccess) return e;
+  const int ctas = shape.sms * shape.resident, blocks = a.outer < ctas ? a.outer : ctas;
   kernel<<<blocks, kColThreads, smem, stream>>>(a);
   return cudaGetLastError();
 }
