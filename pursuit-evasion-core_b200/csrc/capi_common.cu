@@ -30,6 +30,7 @@ int fail(int code, const char *fmt, ...) {
 }
 
 int cuda_fail(cudaError_t err, const char *what) {
+  cudaGetLastError();  // reported here: not again by the next call's check
   const int code =
       err == cudaErrorMemoryAllocation ? PE_ENOMEM : PE_ECUDA;
   return fail(code, "%s: %s", what, cudaGetErrorString(err));

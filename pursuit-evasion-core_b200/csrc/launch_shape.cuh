@@ -50,7 +50,9 @@ inline cudaError_t launch_shape(const void *kernel, int threads, size_t smem,
 // CTAs of one cooperative launch (0: the launch is not possible).
 inline int cooperative_ctas(const void *kernel, int threads, size_t smem) {
   LaunchShape s;
-  return launch_shape(kernel, threads, smem, s) == cudaSuccess ? s.sms * s.resident : 0;
+  if (launch_shape(kernel, threads, smem, s) == cudaSuccess) return s.sms * s.resident;
+  cudaGetLastError();  // the caller reports the refusal
+  return 0;
 }
 
 }  // namespace pe

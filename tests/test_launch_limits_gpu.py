@@ -107,3 +107,14 @@ def test_a_smaller_batch_created_later_leaves_the_limit(precision):
             BatchSolver(narrow, local_precision=precision) as b:
         solve(b)
         np.testing.assert_array_equal(bits(solve(a)), bits(want))
+
+
+def test_a_refused_batch_does_not_fail_the_next_call():
+    """Rows of 2,300 positions exceed the float32 kernel's shared memory; the
+    refusal leaves no error behind for the next handle's first check."""
+    too_wide = [BatchSolve(A3, RelativeGrid(2300, 4, 3, 3, 8.0), 1e-4)]
+    with pytest.raises(ValueError, match="do not fit"):
+        BatchSolver(too_wide, local_precision="float32")
+    with RelativeSolver(A3, RelativeGrid(9, 8, 3, 3, 2.0)) as s:
+        s.initialize()
+        step(s)
