@@ -125,12 +125,37 @@ def train(net, sampler, *, samples=1 << 22, epochs=20, batch=8192, lr=1e-3,
     return losses, time.perf_counter() - started
 
 
+def _depth(obj, name):
+    """Where `obj` takes attribute `name` from: -1 itself, else the place of
+    the class in its method resolution order, None for nowhere."""
+    if name in getattr(obj, "__dict__", ()):
+        return -1
+    for depth, cls in enumerate(type(obj).__mro__):
+        if name in vars(cls):
+            return depth
+    return None
+
+
+def _own_forward(net):
+    """Whether the one-launch kernels compute what `net.forward` does: they
+    take the network, and neither its class nor itself overrides forward."""
+    return (isinstance(net, ValueMLP) and net.fused and "forward" not in net.__dict__
+            and type(net).forward is ValueMLP.forward)
+
+
+def _own_features(sampler):
+    """Whether `sampler.predict` makes the features of `sampler.encode`: an
+    override of encode below the class that brings predict is asked instead."""
+    return (isinstance(sampler, (RelativeNodeSampler, WorldNodeSampler))
+            and _depth(sampler, "predict") <= _depth(sampler, "encode"))
+
+
 def predict_nodes(net, sampler, out, *, chunk=8192):
     """Surrogate value at every grid node into the float32 device tensor `out`."""
     torch = net.torch
     dev = net.dev
     n = sampler.cells
-    if net.fused and chunk > 0 and n > 0 and hasattr(sampler, "predict"):
+    if chunk > 0 and n > 0 and _own_forward(net) and _own_features(sampler):
         direct = (out.dtype == torch.float32 and out.is_contiguous()
                   and out.device == dev and out.dim() == 1 and out.numel() >= n)
         values = out if direct else torch.empty(n, dtype=torch.float32, device=dev)
@@ -163,7 +188,7 @@ def predict_states(net, config, extent, states):
         raise ValueError("query batch exceeds the network's buffers")
     p, e = config.pursuer, config.evader
     lib = _native.library()
-    if net.fused:
+    if _own_forward(net):
         out = torch.empty(n, dtype=torch.float32, device=net.dev)
         _native.check(lib.pe_mlp_predict_relative_states(
             ctypes.byref(net.native_net()), _ptr(states), n, float(extent), float(p.speed_min),
