@@ -158,13 +158,15 @@ def predict_nodes(net, sampler, out, *, chunk=8192):
     if chunk > 0 and n > 0 and _own_forward(net) and _own_features(sampler):
         direct = (out.dtype == torch.float32 and out.is_contiguous()
                   and out.device == dev and out.dim() == 1 and out.numel() >= n)
-        values = out if direct else torch.empty(n, dtype=torch.float32, device=dev)
-        step = 1 << 30  # rows of one launch
+        # rows of one launch; others than a plain float32 table by way of a 16 MB buffer
+        step = min(n, 1 << 30 if direct else 1 << 22)
+        values = None if direct else torch.empty(step, dtype=torch.float32, device=dev)
         for start in range(0, n, step):
             rows = min(step, n - start)
-            sampler.predict(net, start, rows, values[start:start + rows])
-        if not direct:
-            out[:n].copy_(values)
+            piece = out[start:start + rows] if direct else values[:rows]
+            sampler.predict(net, start, rows, piece)
+            if not direct:
+                out[start:start + rows].copy_(piece)
         return out
     chunk = min(chunk, net.batch)
     idx = torch.empty(chunk, dtype=torch.int64, device=dev)

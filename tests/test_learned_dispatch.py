@@ -119,3 +119,26 @@ def test_overridden_forward_is_asked_by_queries(monkeypatch):
     net.native_net = unused
     got = train.predict_states(net, A3, 2.0, torch.zeros(3, 5))
     assert torch.equal(got, torch.full((3,), 7.0))
+
+
+@pytest.mark.parametrize("out", ["double", "strided"])
+def test_results_of_another_layout_go_through_a_bounded_buffer(monkeypatch, out):
+    """A destination that the kernel cannot write directly costs a buffer of at
+    most 32 MB, not one of the whole table."""
+    n = (1 << 23) + 1001
+    pieces = []
+
+    def predict(self, net, first, rows, values):
+        assert values.dtype == torch.float32 and values.is_contiguous() and values.numel() == rows
+        pieces.append((first, rows))
+        values.copy_(torch.arange(first, first + rows))
+
+    monkeypatch.setattr(train.RelativeNodeSampler, "predict", predict)
+    sampler = train.RelativeNodeSampler(A3, GRID)
+    sampler.cells = n
+    table = (torch.zeros(n + 3, dtype=torch.float64) if out == "double"
+             else torch.zeros(n + 3, 2)[:, 1])
+    assert train.predict_nodes(host_net(ValueMLP), sampler, table) is table
+    assert torch.equal(table[:n], torch.arange(n, dtype=table.dtype))
+    assert not table[n:].any()
+    assert max(4 * rows for _, rows in pieces) <= 32 << 20
