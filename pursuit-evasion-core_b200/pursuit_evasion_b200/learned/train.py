@@ -96,6 +96,8 @@ def train(net, sampler, *, samples=1 << 22, epochs=20, batch=8192, lr=1e-3,
         net.adam(lr=lr)
 
     stream = torch.cuda.Stream(device=dev)
+    # the samples, the table and the parameters come from the caller's stream
+    stream.wait_stream(torch.cuda.current_stream(dev))
     graph = None
     losses = []
     started = time.perf_counter()
