@@ -584,8 +584,11 @@ int pe_mlp_gemm_tc(const void *A, const void *B, int M, int N, int K, int lda, i
  * multiples of 8; ldc >= N a multiple of 4. */
 int pe_mlp_gemm_tc_splitk(const void *A, const void *B, int M, int N, int K, int lda, int ldb,
                           int splits, float *C32, int ldc, void *cuda_stream);
-/* Number of pe_mlp_gemm_tc launches whose bounded waits timed out since the
- * last call (then cleared).  Synchronises the device. */
+/* Not 0 if a bounded wait of a tensor-core network kernel (pe_mlp_gemm_tc*,
+ * pe_mlp_forward, pe_mlp_backward, pe_mlp_predict_*) gave up since the last
+ * call (then cleared): a GEMM's output is then incomplete, the outputs of
+ * pe_mlp_forward and pe_mlp_predict_* are NaN in the rows concerned.  Waits for
+ * the null stream; synchronise the launching stream first. */
 int pe_mlp_gemm_tc_timeouts(int32_t *count);
 /* Adam on n FP32 master weights w (w16, if not NULL, receives their bf16
  * copy).  corr[0], corr[1] are the bias corrections 1 - beta^t read on the

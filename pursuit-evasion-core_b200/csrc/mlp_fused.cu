@@ -41,7 +41,8 @@
 // 34 us; backward with all gradients 400, 66, 40 us.
 //
 // Every mbarrier wait is bounded; a wait that gives up sets the error flag
-// of pe_mlp_gemm_tc_timeouts and the CTA still releases its tensor memory.
+// of pe_mlp_gemm_tc_timeouts and the CTA still releases its tensor memory.  The
+// outputs of the rows that it concerns are NaN, and the loss with them.
 #include "mlp_features.cuh"
 #include "mlp_tc.cuh"
 
@@ -550,6 +551,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       // the head, a warp per row: lane l sums columns l, l + 32, ..; a cluster's
       // CTAs take half of the rows each, once both halves of the columns are in
       if (CL == 2 && ok) ok = tile_wait_warp<CL>(&a_ready[t], pass & 1, g.error);
+      // columns of the tile are not there: every output of the CTA becomes NaN
+      if (!ok) wout[lane] = __int_as_float(0x7fc00000);
       asm volatile("bar.sync %0, %1;" ::"r"(1 + t), "n"(32 * WPT) : "memory");
       float w[H / 32];
 #pragma unroll
@@ -567,7 +570,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
         const int64_t out_row = (int64_t)(grp * TPC + t) * TM + rr;
-        if (lane == 0 && ok && out_row < g.rows) {
+        if (lane == 0 && out_row < g.rows) {
           const float out = sum + b_out;
           g.y[out_row] = out;
           if (TRAIN && g.target) {

@@ -307,8 +307,8 @@ int pe_mlp_gemm_tc_splitk(const void *A, const void *B, int M, int N, int K, int
   return PE_OK;
 }
 
-// Timeouts of bounded waits seen by pe_mlp_gemm_tc launches so far (and
-// clear the flag).  Synchronises the device.
+// Whether a bounded wait of the network kernels gave up so far (and clear the
+// flag).
 int pe_mlp_gemm_tc_timeouts(int32_t *count) {
   using namespace pe;
   using namespace pe::tc;

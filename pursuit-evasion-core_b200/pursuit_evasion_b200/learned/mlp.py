@@ -218,6 +218,17 @@ class ValueMLP:
                                                _ptr(self.corr), 1.0, self._stream()))
         self._transpose_weights()
 
+    def check_waits(self):
+        """Synchronise the device; raise if a bounded wait of a network kernel
+        gave up since the last check.  (Inference does not wait for this: the
+        predictions concerned are NaN.)"""
+        self.torch.cuda.synchronize(self.dev)
+        gave_up = ctypes.c_int32()
+        _native.check(self.lib.pe_mlp_gemm_tc_timeouts(ctypes.byref(gave_up)))
+        if gave_up.value:
+            raise _native.NativeError(_native.PE_ETIMEOUT,
+                                      "a bounded device wait of the network kernels gave up")
+
     def set_step(self, step, beta1=0.9, beta2=0.999):
         self.corr.copy_(self.torch.tensor([1 - beta1 ** step, 1 - beta2 ** step],
                                           dtype=self.torch.float32))

@@ -124,7 +124,10 @@ def train(net, sampler, *, samples=1 << 22, epochs=20, batch=8192, lr=1e-3,
             if log:
                 log(f"epoch {epoch + 1}: mse {losses[-1]:.3e}")
     torch.cuda.synchronize(dev)
-    return losses, time.perf_counter() - started
+    seconds = time.perf_counter() - started
+    if hasattr(net, "check_waits"):
+        net.check_waits()
+    return losses, seconds
 
 
 def _depth(obj, name):

@@ -66,3 +66,32 @@ def test_training_waits_for_what_the_caller_queued():
     wait = ("wait", reads[0][1], streams.caller)
     assert wait in streams.log
     assert streams.log.index(wait) < streams.log.index(reads[0])
+
+
+def test_training_checks_the_device_waits_at_its_end():
+    streams = Streams()
+    net = host_net(streams)
+    sampler = SimpleNamespace(cells=100, encode=lambda *args: streams.log.append(("read",)))
+    train.train(net, sampler, samples=128, epochs=2, batch=64, use_graph=False)
+    assert streams.log[-1] == ("check",) and streams.log.count(("read",)) == 4
+
+
+@pytest.mark.parametrize("gave_up", [0, 1])
+def test_a_wait_that_gave_up_is_raised(gave_up):
+    from pursuit_evasion_b200 import _native
+    from pursuit_evasion_b200.learned.mlp import ValueMLP
+
+    def timeouts(count):
+        count._obj.value = gave_up
+        return 0
+
+    streams = Streams()
+    net = ValueMLP.__new__(ValueMLP)
+    net.torch, net.dev = streams, torch.device("cpu")
+    net.lib = SimpleNamespace(pe_mlp_gemm_tc_timeouts=timeouts)
+    if gave_up:
+        with pytest.raises(_native.NativeError, match="gave up"):
+            net.check_waits()
+    else:
+        net.check_waits()
+    assert streams.log == [("synchronize",)]
