@@ -11,7 +11,7 @@
 // heading axis' are carried from step to step, the x axis' shared inside the
 // chunk, and the range checks are replaced by one test of the result
 // (relative5d_exact_walk.cuh): about 165 double operations per cell, which
-// bound it (64 per clock and SM): 1.77 ms per stage at 65x48x21x21 (4.0 ms
+// bound it (64 per clock and SM): 1.82 ms per stage at 65x48x21x21 (4.0 ms
 // for the thread-per-cell kernel), of which the double operations are 0.85.
 #include "launch_shape.cuh"
 #include "relative5d_exact_walk.cuh"
@@ -22,16 +22,27 @@ namespace {
 
 using namespace ring;
 
+// The spacings' constants are made on the host: as kernel parameters they are
+// operands in the constant bank, where 20 doubles made in the kernel took
+// registers of the 128 that two CTAs per SM leave a thread (RK2 step of
+// 33x24x11x11 0.208 -> 0.202 ms, 57x36x17x17 1.75 -> 1.67, 64x48x21x21 3.33 ->
+// 3.24).  65x48x21x21 takes 3.63 ms: 3.78 before, and 3.59 in a variant compiled
+// for its row pitch and 13 rows, which no other grid could use.
+struct WalkArgs {
+  RingArgs ring;
+  exact::AxisSteps st;
+};
+
 // heading (cos, sin) pairs and x positions, in double
 __host__ __device__ inline int table_bytes(const Rel5Grid &g) { return 16 * g.nh + 8 * g.xp; }
 
-template <int ORDER, int BLEND, int XR, int XPC, int RC, bool OVERLAP>
+template <int ORDER, int BLEND, int XR, bool OVERLAP>
 __global__ void __launch_bounds__(TARGET_THREADS, 2)
-    rel5_walk_exact_kernel(const __grid_constant__ RingArgs a) {
+    rel5_walk_exact_kernel(const __grid_constant__ WalkArgs args) {
+  const RingArgs &a = args.ring;
   extern __shared__ __align__(128) float smem[];
   const Rel5Grid &g = a.g;
-  const int R = RC ? RC : a.rows, XP = XPC ? XPC : g.xp;
-  const int XC = XPC ? XPC / 4 : a.xc;
+  const int R = a.rows, XP = g.xp, XC = a.xc;
   const SmemLayout L = smem_layout(R, XP, table_bytes(g));
   float *own = smem + L.own_off;  // [8][R+4][XP]
   float *nbr = smem + L.nb_off;   // [2][9][R][XP]
@@ -76,10 +87,7 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
     constexpr int KP = (XR + 2) & 3, IEND = (XR + 3) & 3;
     const bool kend = x0 == g.nx - 2 - KP, iend = x0 == g.nx - 1 - IEND;
     const int valid = iend ? IEND + 1 : 4;
-    const exact::AxisSteps st{exact::axis_step(g.dx, g.rdx, g.rdx2),
-                              exact::axis_step(g.dphi, g.rdphi, g.rdphi2),
-                              exact::axis_step(g.dvp, g.rdvp, g.rdvp2),
-                              exact::axis_step(g.dve, g.rdve, g.rdve2)};
+    const exact::AxisSteps &st = args.st;
     const int ctr = (r + 2) * XP + x0;  // this chunk in an own slot
     const int nbo = r * XP + x0;        // this chunk in a neighbour slot
     bool alive = true;
@@ -154,33 +162,34 @@ __global__ void __launch_bounds__(TARGET_THREADS, 2)
   }
 }
 
-template <int ORDER, int BLEND, int XR, int XPC = 0, int RC = 0, bool OVERLAP = false>
+template <int ORDER, int BLEND, int XR, bool OVERLAP>
 cudaError_t launch_xr(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
-  auto kernel = rel5_walk_exact_kernel<ORDER, BLEND, XR, XPC, RC, OVERLAP>;
+  auto kernel = rel5_walk_exact_kernel<ORDER, BLEND, XR, OVERLAP>;
   static thread_local LaunchShape shape;
   const cudaError_t e =
       launch_shape(reinterpret_cast<const void *>(kernel), threads, smem, shape);
   if (e != cudaSuccess) return e;
-  return launch_overlapped(OVERLAP, kernel,
-                           dim3((unsigned)std::min(args.items, shape.sms * shape.resident)), threads,
-                           smem,
-                           stream, args);
+  const int ctas = std::min(args.items, shape.sms * shape.resident);
+  const Rel5Grid &g = args.g;
+  const WalkArgs walk{args, exact::AxisSteps{exact::axis_step(g.dx, g.rdx, g.rdx2),
+                                             exact::axis_step(g.dphi, g.rdphi, g.rdphi2),
+                                             exact::axis_step(g.dvp, g.rdvp, g.rdvp2),
+                                             exact::axis_step(g.dve, g.rdve, g.rdve2)}};
+  return launch_overlapped(OVERLAP, kernel, dim3((unsigned)ctas), threads, smem, stream, walk);
 }
 
 template <int ORDER, int BLEND, bool OVERLAP>
 cudaError_t launch_nx(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
   switch (args.g.nx & 3) {
-    case 0: return launch_xr<ORDER, BLEND, 0, 0, 0, OVERLAP>(args, smem, threads, stream);
-    case 1: return launch_xr<ORDER, BLEND, 1, 0, 0, OVERLAP>(args, smem, threads, stream);
-    case 2: return launch_xr<ORDER, BLEND, 2, 0, 0, OVERLAP>(args, smem, threads, stream);
-    default: return launch_xr<ORDER, BLEND, 3, 0, 0, OVERLAP>(args, smem, threads, stream);
+    case 0: return launch_xr<ORDER, BLEND, 0, OVERLAP>(args, smem, threads, stream);
+    case 1: return launch_xr<ORDER, BLEND, 1, OVERLAP>(args, smem, threads, stream);
+    case 2: return launch_xr<ORDER, BLEND, 2, OVERLAP>(args, smem, threads, stream);
+    default: return launch_xr<ORDER, BLEND, 3, OVERLAP>(args, smem, threads, stream);
   }
 }
 
 template <int ORDER, int BLEND>
 cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t stream) {
-  if (args.g.xp == 68 && args.g.nx == 65 && args.rows == 13 && !args.overlap)
-    return launch_xr<ORDER, BLEND, 1, 68, 13>(args, smem, threads, stream);
   return args.overlap ? launch_nx<ORDER, BLEND, true>(args, smem, threads, stream)
                       : launch_nx<ORDER, BLEND, false>(args, smem, threads, stream);
 }
