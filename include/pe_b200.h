@@ -152,13 +152,18 @@ int pe_host_free(void *ptr);
 int pe_relative_device_field(pe_relative *h, float **device_field);
 int pe_relative_row_pitch(const pe_relative *h, int32_t *floats);
 
-/* Tile shape of the float32 stage kernel: a CTA owns `rows` y rows of one
+/* Tile shape of the tiled stage kernels (float32, and float64 where its tiled
+ * kernel runs): a CTA owns `rows` y rows of one
  * (vP, vE) pair and sweeps `psi_chunk` headings.  (0, 0) restores the
  * default; shapes that exceed the kernel's thread or shared-memory limits
  * are rejected with PE_EINVAL.  Results do not depend on the tile. */
 int pe_relative_set_tile(pe_relative *h, int32_t rows, int32_t psi_chunk);
 int pe_relative_get_tile(const pe_relative *h, int32_t *rows,
                          int32_t *psi_chunk);
+
+/* Whether the handle's float64 stages run the tiled kernel with its tile (0:
+ * a cell per thread, and float32 handles).  Results do not depend on it. */
+int pe_relative_exact_tiled(const pe_relative *h, int32_t *tiled);
 
 /* Launch shape of the float32 stage kernel for the handle's tile: threads
  * per CTA, dynamic shared memory per CTA, and CTAs resident per SM at the
@@ -437,6 +442,9 @@ int pe_world_copy_field(pe_world *h, float *host_field);
 int pe_world_copy_arrival(pe_world *h, float *host_arrival);
 /* max |V_new - V_old| of the most recent step. */
 int pe_world_residual(pe_world *h, double *residual);
+/* Whether the exact stages run the column kernel (0: a cell per thread, and
+ * fast handles).  Results do not depend on it. */
+int pe_world_exact_column(const pe_world *h, int32_t *column);
 int pe_world_set_stream(pe_world *h, void *cuda_stream);
 int pe_world_profile(pe_world *h, int enable);
 int pe_world_kernel_time(pe_world *h, double *total_ms, int64_t *launches);

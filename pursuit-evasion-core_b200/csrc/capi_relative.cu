@@ -482,6 +482,15 @@ int pe_relative_get_tile(const pe_relative *h, int32_t *rows,
   return PE_OK;
 }
 
+int pe_relative_exact_tiled(const pe_relative *h, int32_t *tiled) {
+  if (!h || !tiled) return fail(PE_EINVAL, "NULL argument");
+  pe::Rel5Stage s{};
+  s.src = h->a;
+  s.dst = h->b;
+  *tiled = h->p.precision == PE_LOCAL_F64 && pe::rel5_walk_exact_applies(h->g, h->tile, s);
+  return PE_OK;
+}
+
 int pe_relative_kernel_info(const pe_relative *h, int32_t *threads,
                             int32_t *smem_bytes, int32_t *resident_ctas) {
   if (!h) return fail(PE_EINVAL, "handle is NULL");

@@ -447,6 +447,12 @@ int pe_world_residual(pe_world *h, double *residual) {
   return PE_OK;
 }
 
+int pe_world_exact_column(const pe_world *h, int32_t *column) {
+  if (!h || !column) return fail(PE_EINVAL, "NULL argument");
+  *column = h->column;
+  return PE_OK;
+}
+
 int pe_world_set_stream(pe_world *h, void *cuda_stream) {
   int rc = enter(h);
   if (rc) return rc;

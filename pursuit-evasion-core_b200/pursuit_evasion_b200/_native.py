@@ -199,6 +199,7 @@ SIGNATURES = {
     "pe_relative_set_tile": (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_int32]),
     "pe_relative_get_tile": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int32),
                                             ctypes.POINTER(ctypes.c_int32)]),
+    "pe_relative_exact_tiled": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int32)]),
     "pe_relative_kernel_info": (ctypes.c_int, [_P] + [ctypes.POINTER(ctypes.c_int32)] * 3),
     "pe_relative_stats": (ctypes.c_int, [_P, _DP, _DP]),
     "pe_relative_profile": (ctypes.c_int, [_P, ctypes.c_int]),
@@ -308,6 +309,7 @@ SIGNATURES = {
     "pe_world_copy_field": (ctypes.c_int, [_P, _P]),
     "pe_world_copy_arrival": (ctypes.c_int, [_P, _P]),
     "pe_world_residual": (ctypes.c_int, [_P, _DP]),
+    "pe_world_exact_column": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int32)]),
     "pe_world_set_stream": (ctypes.c_int, [_P, _P]),
     "pe_world_profile": (ctypes.c_int, [_P, ctypes.c_int]),
     "pe_world_kernel_time": (ctypes.c_int, [_P, _DP, _I64P]),

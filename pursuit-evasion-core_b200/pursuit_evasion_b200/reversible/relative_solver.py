@@ -206,7 +206,7 @@ class RelativeSolver:
 
     @property
     def tile(self):
-        """(rows, psi_chunk) of the float32 stage kernel."""
+        """(rows, psi_chunk) of the tiled stage kernels."""
         rows, chunk = ctypes.c_int32(), ctypes.c_int32()
         _native.check(self._lib.pe_relative_get_tile(self._h, ctypes.byref(rows),
                                                      ctypes.byref(chunk)))
@@ -215,6 +215,13 @@ class RelativeSolver:
     def set_tile(self, rows, psi_chunk):
         _native.check(self._lib.pe_relative_set_tile(self._h, int(rows),
                                                      int(psi_chunk)))
+
+    @property
+    def exact_tiled(self):
+        """Whether float64 stages run the tiled kernel (else a cell per thread)."""
+        tiled = ctypes.c_int32()
+        _native.check(self._lib.pe_relative_exact_tiled(self._h, ctypes.byref(tiled)))
+        return bool(tiled.value)
 
     def kernel_info(self):
         """(threads per CTA, shared bytes per CTA, resident CTAs per SM)."""

@@ -222,6 +222,13 @@ class WorldSolver:
         _native.check(self._lib.pe_world_copy_arrival(self._h, out.ctypes.data))
         return out.reshape(self.shape)
 
+    @property
+    def exact_column(self):
+        """Whether exact stages run the column kernel (else a cell per thread)."""
+        column = ctypes.c_int32()
+        _native.check(self._lib.pe_world_exact_column(self._h, ctypes.byref(column)))
+        return bool(column.value)
+
     def residual(self):
         r = ctypes.c_double()
         _native.check(self._lib.pe_world_residual(self._h, ctypes.byref(r)))
