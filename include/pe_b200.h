@@ -442,8 +442,10 @@ int pe_world_copy_field(pe_world *h, float *host_field);
 int pe_world_copy_arrival(pe_world *h, float *host_arrival);
 /* max |V_new - V_old| of the most recent step. */
 int pe_world_residual(pe_world *h, double *residual);
-/* Whether the exact stages run the column kernel (0: a cell per thread, and
- * fast handles).  Results do not depend on it. */
+/* Whether the next exact stage runs the column kernel (0: a cell per thread, and
+ * fast handles): it takes 3 to 8 evader speeds, blocks that fit shared memory,
+ * and fields in which the last synchronising call found no nonzero value below
+ * 2^-70.  Results do not depend on it. */
 int pe_world_exact_column(const pe_world *h, int32_t *column);
 int pe_world_set_stream(pe_world *h, void *cuda_stream);
 int pe_world_profile(pe_world *h, int enable);

@@ -224,7 +224,7 @@ class WorldSolver:
 
     @property
     def exact_column(self):
-        """Whether exact stages run the column kernel (else a cell per thread)."""
+        """Whether the next exact stage runs the column kernel (else a cell per thread)."""
         column = ctypes.c_int32()
         _native.check(self._lib.pe_world_exact_column(self._h, ctypes.byref(column)))
         return bool(column.value)

@@ -9,7 +9,7 @@ from pursuit_evasion_b200.reversible.free_dp import RelativeGrid
 from pursuit_evasion_b200.reversible.relative_solver import RelativeSolver
 from pursuit_evasion_b200.reversible.world_dp import WorldGrid, WorldSolver
 from tests import oracle_lib
-from tests.helpers import A3, CONFIG1_GRID, CONFIG2_GRID
+from tests.helpers import A3, CONFIG1_GRID, CONFIG2_GRID, bits
 from tests.test_relative_tiled_exact_gpu import GRIDS
 from tests.test_recomputed_cells_gpu import RELATIVE_GRIDS
 from tests.test_world_column_exact_gpu import initial
@@ -71,3 +71,48 @@ def test_world_cell_per_thread_stage_equals_the_oracle(oracle, order, boundary, 
     np.testing.assert_array_equal(np.isnan(got), np.isnan(arrival))
     held = ~np.isnan(arrival)
     np.testing.assert_array_equal(got[held], arrival[held])
+
+
+@pytest.mark.parametrize("boundary", ["linear", "legacy_signed"])
+def test_world_fields_with_tiny_values_change_kernels(oracle, boundary):
+    """Values below 2^-70 that the field starts with, or that a check finds, move
+    the stages to a cell per thread, and back once they are gone; the results
+    are the oracle's throughout.  Between checks the column kernel itself takes
+    the general arithmetic."""
+    grid = WorldGrid(7, 4, 3, 5, 3.5)
+    p, e = A3.pursuer, A3.evader
+    cfg = oracle_lib.W8Cfg(grid.positions, grid.headings, grid.p_speeds, grid.e_speeds, 2,
+                           int(boundary == "linear"), 1, grid.extent, A3.arena_half_width,
+                           A3.capture_radius, p.speed_min, p.speed_max, e.speed_min,
+                           e.speed_max, p.acceleration, e.acceleration, p.max_curvature,
+                           e.max_curvature, 0.8)
+
+    def tiny(v):
+        return bool(((v != 0) & (np.abs(v) < 2.0 ** -70)).any())
+
+    with WorldSolver(A3, grid, speed_boundary=boundary) as s:
+        dt = np.float32(s.dt_limit).item()
+        for kind, check in (("noise", True), ("tiny", True), ("bound", True), ("bound", False),
+                            ("one", True)):
+            a = initial("noise" if kind == "one" else kind, grid.states)
+            if kind == "one":
+                a[a.size // 2] = 1e-30
+            b = np.zeros_like(a)
+            arrival = np.where(a <= 0, np.float32(0), np.float32(np.nan)).astype(np.float32)
+            s.init_field(a)
+            assert s.exact_column == (not tiny(a))
+            tau, seen = 0.0, []
+            for _ in range(4):
+                s.step(dt)
+                oracle.w8_stage(cfg, a, b, None, arrival, dt, tau)
+                oracle.w8_stage(cfg, b, a, a, arrival, dt, tau)
+                tau += dt
+                if check:
+                    s.synchronize()
+                    seen.append(tiny(a))
+                    assert s.exact_column == (not seen[-1])
+            np.testing.assert_array_equal(bits(s.field().reshape(-1)), bits(a))
+            got = s.arrival().reshape(-1)
+            np.testing.assert_array_equal(np.isnan(got), np.isnan(arrival))
+            if kind in ("noise", "one"):
+                assert s.exact_column
