@@ -354,6 +354,9 @@ int pe_batch_create(const pe_relative_params *params, const double *horizons,
  * Results do not depend on the tile. */
 int pe_batch_set_tile(pe_batch *h, int32_t solve, int32_t rows);
 int pe_batch_get_tile(const pe_batch *h, int32_t solve, int32_t *rows);
+/* Whether a float64 batch runs the tiled kernel (0: a cell per thread, and
+ * float32 batches).  Results do not depend on it. */
+int pe_batch_exact_tiled(const pe_batch *h, int32_t *tiled);
 int pe_batch_set_stream(pe_batch *h, void *cuda_stream);
 /* Capture field and arrival of every solve at t = 0. */
 int pe_batch_init(pe_batch *h);

@@ -120,6 +120,55 @@ int exact_chunk_cap(const pe_batch *h, int ctas) {
   return best;
 }
 
+// Rows per item of the cell-per-thread kernel: about a CTA's 256 cells.
+int cell_rows(int nx) {
+  return std::max(1, std::min(nx, (pe::kRel5BatchThreads + nx - 1) / nx));
+}
+
+// Whether an exact batch is faster in the tiled kernel, by the estimated stage
+// times of both over the run, in microseconds on a B200 (296 and 592 CTAs).  A
+// CTA of the tiled kernel has a thread per 4 cells of one speed pair's rows, so
+// small planes fill few of its warps, and a heading step takes 3.6 us however few
+// they are (0.3 us more per warp); its stage is bound by the sum of the items,
+// by the longest, or by the waves they make.  The cell-per-thread kernel takes
+// 5.8 us per pass over 256 cells and 2.1 us per 256 cells.  Fitted to 254 batches of
+// 1-16 grids of 5-50 positions, 4-60 headings and 3-23 speeds, residuals 6 and 10 %:
+// none is more than 3 % slower than in the cell-per-thread kernel, two than in
+// the tiled one.  A solve of 12x5x14x4 takes 168 us tiled and 77 us here, four of
+// 17-49 positions 22.7 and 56 ms.
+bool tiled_is_faster(const pe_batch *h) {
+  const int cap = exact_chunk_cap(h, 2 * 148);
+  double tiled = 0, cells = 0;
+  double items = 0, work = 0, longest = 0, cell_work = 0, cell_longest = 0;
+  for (int pos = 0; pos < h->count; pos++) {
+    const int i = h->order[pos];
+    const pe::Rel5Grid &g = h->grids[i];
+    const double pairs = (double)g.nvp * g.nve;
+    const int rows = pe::rel5_batch_tiled_rows(g.nx, g.xp, h->rows[i]);
+    const int chunks = (g.nh + cap - 1) / cap, chunk = (g.nh + chunks - 1) / chunks;
+    const int warps = (rows * (g.xp / 4) + 31) / 32;
+    const double count = pairs * ((g.nh + chunk - 1) / chunk) * ((g.nx + rows - 1) / rows);
+    const double item = (chunk + 1) * (3.6 + 0.31 * warps);
+    items += count;
+    work += count * item;
+    longest = std::max(longest, item);
+    for (int y = 0, r = cell_rows(g.nx); y < g.nx; y += r) {
+      const int n = std::min(r, g.nx - y) * g.nx;
+      const double cell_item = 5.8 * ((n + pe::kRel5BatchThreads - 1) / pe::kRel5BatchThreads) +
+                               2.1 * n / pe::kRel5BatchThreads;
+      cell_work += pairs * g.nh * cell_item;
+      cell_longest = std::max(cell_longest, cell_item);
+    }
+    // solves still stepping at step k are a prefix
+    const size_t after = pos + 1 < h->count ? h->steps[h->order[pos + 1]].size() : 0;
+    const double stages = 2.0 * (double)(h->steps[i].size() - after);
+    tiled += stages * (3.1 + std::max({work / 296, longest,
+                                       0.92 * work / items * std::ceil(items / 296)}));
+    cells += stages * (8.6 + cell_work / 592 + 0.22 * cell_longest);
+  }
+  return tiled < 0.95 * cells;
+}
+
 // Descriptors and the active-item prefix for the current tiles.
 int upload_descriptors(pe_batch *h) {
   std::vector<pe::Rel5BatchSolve> d(h->count);
@@ -286,13 +335,19 @@ int pe_batch_create(const pe_relative_params *params, const double *horizons, in
     h->plane_off.push_back(planes);
     planes += (size_t)g.nx * g.nx;
   }
-  // exact rows wider than a CTA's threads take a cell per thread
-  h->tiled = !(h->exact && h->wide);
   h->order.resize(count);
   std::iota(h->order.begin(), h->order.end(), 0);
   std::stable_sort(h->order.begin(), h->order.end(), [&](int x, int y) {
     return h->steps[x].size() > h->steps[y].size();
   });
+  // exact rows wider than a CTA's threads, and batches of small planes, take a
+  // cell per thread
+  if (h->exact && h->wide) {
+    h->tiled = false;
+  } else if (h->exact && !tiled_is_faster(h)) {
+    h->tiled = false;
+    for (int i = 0; i < count; i++) h->rows[i] = cell_rows(h->grids[i].nx);
+  }
 
   cudaError_t err = cudaSuccess;
   auto take = [&](cudaError_t e) {
@@ -360,6 +415,12 @@ int pe_batch_set_tile(pe_batch *h, int32_t solve, int32_t rows) {
     return fail(PE_EINVAL, "rows must be in [1, positions]");
   h->rows[solve] = rows;
   return upload_descriptors(h);
+}
+
+int pe_batch_exact_tiled(const pe_batch *h, int32_t *tiled) {
+  if (!h || !tiled) return fail(PE_EINVAL, "handle or tiled is NULL");
+  *tiled = h->exact && h->tiled;
+  return PE_OK;
 }
 
 int pe_batch_get_tile(const pe_batch *h, int32_t solve, int32_t *rows) {

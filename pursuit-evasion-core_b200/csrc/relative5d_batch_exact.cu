@@ -1,9 +1,10 @@
 // Batched relative 5D solves with the exact cell update (double local
 // arithmetic in the reference executable's order, relative5d_exact.cuh):
 // every solve of a batch reproduces the reference executable bit for bit.
-// This file is compiled with -fmad=false.  Only batches with rows of more than
-// 1,024 positions come here: a row of the tiled kernel
-// (relative5d_batch_tiled_exact.cu) has at most 256 4-cell chunks.
+// This file is compiled with -fmad=false.  Batches of small planes come here,
+// where the tiled kernel (relative5d_batch_tiled_exact.cu) fills few of a CTA's
+// warps (tiled_is_faster in capi_batch.cu), and batches with rows of more than
+// 1,024 positions: a row of the tiled kernel has at most 256 4-cell chunks.
 #include "relative5d_batch_impl.cuh"
 #include "relative5d_exact.cuh"
 

@@ -236,6 +236,7 @@ SIGNATURES = {
     "pe_batch_create": (ctypes.c_int, [ctypes.POINTER(RelativeParams), _DP, ctypes.c_int32,
                                        ctypes.c_int32, ctypes.POINTER(ctypes.c_void_p)]),
     "pe_batch_set_tile": (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_int32]),
+    "pe_batch_exact_tiled": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int32)]),
     "pe_batch_get_tile": (ctypes.c_int, [_P, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32)]),
     "pe_batch_set_stream": (ctypes.c_int, [_P, _P]),
     "pe_batch_init": (ctypes.c_int, [_P]),

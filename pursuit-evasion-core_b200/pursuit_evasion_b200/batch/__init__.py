@@ -165,6 +165,13 @@ class BatchSolver:
         _native.check(self._lib.pe_batch_get_tile(self._h, int(solve), ctypes.byref(r)))
         return r.value
 
+    @property
+    def exact_tiled(self):
+        """Whether a float64 batch runs the tiled kernel (else a cell per thread)."""
+        tiled = ctypes.c_int32()
+        _native.check(self._lib.pe_batch_exact_tiled(self._h, ctypes.byref(tiled)))
+        return bool(tiled.value)
+
     def set_stream(self, stream_ptr):
         _native.check(self._lib.pe_batch_set_stream(self._h, stream_ptr))
 
