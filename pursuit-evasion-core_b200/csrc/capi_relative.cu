@@ -156,7 +156,7 @@ int pe_relative_create(const pe_relative_params *params, pe_relative **out) {
   h->p = *params;
   h->g = make_grid(params);
   h->limit = cfl_limit(params, h->g);
-  h->tile = pe::rel5_default_tile(h->g);
+  h->tile = pe::rel5_default_tile(h->g, h->p.precision == PE_LOCAL_F64);
   const size_t bytes = sizeof(float) * (size_t)h->g.n_padded;
   const int nh = h->g.nh;
   std::vector<double> sn(nh), cs(nh);
@@ -466,7 +466,7 @@ int pe_relative_set_tile(pe_relative *h, int32_t rows, int32_t psi_chunk) {
   int rc = enter(h);
   if (rc) return rc;
   pe::Rel5Tile t{rows, psi_chunk};
-  if (rows == 0 && psi_chunk == 0) t = pe::rel5_default_tile(h->g);
+  if (rows == 0 && psi_chunk == 0) t = pe::rel5_default_tile(h->g, h->p.precision == PE_LOCAL_F64);
   if (!pe::rel5_tile_valid(h->g, t))
     return fail(PE_EINVAL, "tile rows=%d psi_chunk=%d does not fit this grid",
                 rows, psi_chunk);

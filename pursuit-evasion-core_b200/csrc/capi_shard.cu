@@ -114,7 +114,7 @@ int pe_relative_shard_create(const pe_relative_params *params, int32_t vp_begin,
   h->g.own_n = vp_end - vp_begin;
   h->g.slab_lo = h->lo;
   h->slab_floats = h->g.sv;
-  h->tile = pe::rel5_default_tile(h->g);
+  h->tile = pe::rel5_default_tile(h->g, h->p.precision == PE_LOCAL_F64);
   const int slabs = h->hi - h->lo, nh = h->g.nh;
   const size_t bytes = sizeof(float) * (size_t)h->g.sv * slabs;
   std::vector<double> sn(nh), cs(nh);

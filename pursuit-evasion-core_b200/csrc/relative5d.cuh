@@ -82,10 +82,10 @@ struct Rel5Tile {
 // Shared memory the fast kernel needs for a tile.
 size_t rel5_fast_smem_bytes(const Rel5Grid &g, const Rel5Tile &t);
 
-// Default tile for a grid: the one of least estimated stage time.
-Rel5Tile rel5_default_tile(const Rel5Grid &g);
+// Default tile of the float32 or the exact stage.
+Rel5Tile rel5_default_tile(const Rel5Grid &g, bool exact);
 
-// Estimated time of one float32 stage in tiles `t`, microseconds.
+// Rough time of one float32 stage in tiles `t`, microseconds.
 double rel5_tile_cost(const Rel5Grid &g, const Rel5Tile &t);
 
 // Resident CTAs per SM of the most recent fast-stage launch.

@@ -547,43 +547,57 @@ size_t rel5_fast_smem_bytes(const Rel5Grid &g, const Rel5Tile &t) {
   return (size_t)smem_layout(t.rows, g.xp, 8 * g.nh).bytes;
 }
 
-// Time of one stage in tiles `t`, in microseconds of the float32 kernel on a
-// B200: the items' heading steps (each item also pays about 3 steps to start
-// its rings) over the CTAs that fit the SMs by shared memory and registers.
-// A step of the CTAs of one SM costs 0.1 us per consumer warp (throughput),
-// and not less than 0.9 us (the latency of one step); the y halo rows add a
-// little (17-row items beat 7-row ones by 6 % at 49x36x15x15).  Measured stages lie
-// within 20 % of it from 16,200 to 89 M cells.
-double rel5_tile_cost(const Rel5Grid &g, const Rel5Tile &t) {
-  const int kSms = 148, kRegs = 128;
-  const int warps = (t.rows * (g.xp / 4) + 31) / 32;
+namespace {
+
+// How the items of a stage in tiles `t` fall on the SMs: CTAs that fit one by
+// shared memory and registers, rounds that fill all of them, items of the last.
+struct TileWaves {
+  int warps, resident;
+  int64_t full, rest;
+};
+constexpr int kSms = 148;
+
+TileWaves tile_waves(const Rel5Grid &g, const Rel5Tile &t) {
+  const int kRegs = 128;
+  TileWaves w;
+  w.warps = (t.rows * (g.xp / 4) + 31) / 32;
   const int smem = (int)rel5_fast_smem_bytes(g, t) + 1024;
-  const int resident = std::max(
-      1, std::min({227 * 1024 / smem, 65536 / (kRegs * 32 * (warps + 1)), 32}));
+  w.resident =
+      std::max(1, std::min({227 * 1024 / smem, 65536 / (kRegs * 32 * (w.warps + 1)), 32}));
   const int64_t slabs = (g.nx + t.rows - 1) / t.rows;
   const int64_t chunks = (g.nh + t.psi_chunk - 1) / t.psi_chunk;
   const int64_t items = slabs * g.nve * (g.own_n > 0 ? g.own_n : g.nvp) * chunks;
-  auto step = [&](int64_t ctas) { return std::max(0.9, 0.1 * warps * (double)ctas); };
-  const int64_t full = items / (kSms * resident), rest = items % (kSms * resident);
-  return (t.psi_chunk + 3) * (1 + 0.3 / t.rows) *
-         (full * step(resident) + (rest ? step((rest + kSms - 1) / kSms) : 0.0));
+  w.full = items / (kSms * w.resident);
+  w.rest = items % (kSms * w.resident);
+  return w;
 }
 
-// The tile of least rel5_tile_cost, the larger one where two cost the same
-// (fewer halo rows).  Heading chunks stay at 24 or below: the CTAs resident
-// at a time then share the planes of a few headings in L2 (at 65x48x21x21
-// chunks of 48 measured 3 % slower than 24).  The rule before this took the
-// rows with the fewest idle rows at 24 headings: it gave one-row items on 41
-// positions (534 us per RK2 step, 156 us now) and left most SMs idle on small
-// grids (17x12x7x7: one item per speed pair, 17 us per stage, 8 us now).
-Rel5Tile rel5_default_tile(const Rel5Grid &g) {
+// Time of one float32 stage in tiles `t`, launch included: a heading step of
+// one CTA takes 0.78 us and 0.05 us per consumer warp, each further CTA of the SM
+// adds 0.034 us and 0.045 us per warp; an item also pays 0.73 steps to start its
+// rings.  Fitted to 3,400 (grid, tile) pairs of 3e3 to 5e7 cells, residual 6 %.
+double stage_time_f32(const Rel5Grid &g, const Rel5Tile &t) {
+  const TileWaves w = tile_waves(g, t);
+  auto step = [&](int64_t ctas) {
+    return 0.78 + 0.049 * w.warps + (0.045 * w.warps + 0.034) * (double)(ctas - 1);
+  };
+  return 5.6 + (t.psi_chunk + 0.73) *
+                   (w.full * step(w.resident) + (w.rest ? step((w.rest + kSms - 1) / kSms) : 0.0));
+}
+
+// The valid tile of least `time`, the larger one where two cost the same (fewer
+// halo rows).  Heading chunks stay at 24 or below: the CTAs resident at a time
+// then share the planes of a few headings in L2 (at 65x48x21x21 chunks of 48
+// measured 3 % slower than 24).
+template <class Time>
+Rel5Tile cheapest_tile(const Rel5Grid &g, Time time) {
   Rel5Tile best{1, std::min(g.nh, 24)};
   double best_cost = 1e300;
   for (int rows = 1; rows <= g.nx; rows++)
     for (int chunks = 1; chunks <= g.nh / MIN_ITEM_STEPS; chunks++) {
       const Rel5Tile t{rows, (g.nh + chunks - 1) / chunks};
       if (t.psi_chunk > 24 || !rel5_tile_valid(g, t)) continue;
-      const double cost = rel5_tile_cost(g, t);
+      const double cost = time(g, t);
       if (cost < best_cost * (1 - 1e-9) ||
           (cost < best_cost * (1 + 1e-9) &&
            t.rows * t.psi_chunk >= best.rows * best.psi_chunk)) {
@@ -592,6 +606,49 @@ Rel5Tile rel5_default_tile(const Rel5Grid &g) {
       }
     }
   return best;
+}
+
+// Up to 7 consumer warps with the fewest idle rows, most rows of these, and
+// equal heading chunks of about 24.
+Rel5Tile widest_even_tile(const Rel5Grid &g) {
+  Rel5Tile t{1, 1};
+  int least_idle = 1 << 30;
+  for (int rows = 1; rows * (g.xp / 4) <= TARGET_THREADS - 32 && rows <= g.nx; rows++) {
+    const int idle = (g.nx + rows - 1) / rows * rows - g.nx;
+    if (idle <= least_idle) {
+      least_idle = idle;
+      t.rows = rows;
+    }
+  }
+  const int chunks = (g.nh + 23) / 24;
+  t.psi_chunk = (g.nh + chunks - 1) / chunks;
+  return t;
+}
+
+}  // namespace
+
+// A coarser estimate in the same units, which the rules between kernels and
+// launch forms were measured with: 0.1 us per consumer warp and CTA, and not less
+// than 0.9 us, per step; 3 steps to start an item; 0.3 / rows for the halo rows.
+double rel5_tile_cost(const Rel5Grid &g, const Rel5Tile &t) {
+  const TileWaves w = tile_waves(g, t);
+  auto step = [&](int64_t ctas) { return std::max(0.9, 0.1 * w.warps * (double)ctas); };
+  return (t.psi_chunk + 3) * (1 + 0.3 / t.rows) *
+         (w.full * step(w.resident) + (w.rest ? step((w.rest + kSms - 1) / kSms) : 0.0));
+}
+
+// Exact: the tile of least rel5_tile_cost.  Float32: the widest even tile, unless
+// another is estimated to be over 8 % faster (41x30x13x13 537 us per RK2 step in
+// the even tile's single rows, 165 in the other; 17x12x7x7, one item per speed
+// pair, 35 and 19).  Of 714 random grids 4 are more than 2 % behind the even tile,
+// 6 % at most; chosen by rel5_tile_cost alone 57 of 700 were, the worst by 21 %,
+// and the average step took 2.3 % longer.
+Rel5Tile rel5_default_tile(const Rel5Grid &g, bool exact) {
+  if (exact) return cheapest_tile(g, rel5_tile_cost);
+  const Rel5Tile even = widest_even_tile(g), other = cheapest_tile(g, stage_time_f32);
+  return rel5_tile_valid(g, even) && stage_time_f32(g, even) < 1.08 * stage_time_f32(g, other)
+             ? even
+             : other;
 }
 
 bool rel5_tile_valid(const Rel5Grid &g, const Rel5Tile &t) {
