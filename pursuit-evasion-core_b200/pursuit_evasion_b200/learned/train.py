@@ -151,6 +151,8 @@ def _own_forward(net):
 def _own_features(sampler):
     """Whether `sampler.predict` makes the features of `sampler.encode`: an
     override of encode below the class that brings predict is asked instead."""
+    if type(sampler) in (RelativeNodeSampler, WorldNodeSampler):
+        return "encode" not in sampler.__dict__ or "predict" in sampler.__dict__
     return (isinstance(sampler, (RelativeNodeSampler, WorldNodeSampler))
             and _depth(sampler, "predict") <= _depth(sampler, "encode"))
 
