@@ -10,8 +10,10 @@
 // chunks keep a batch of few solves spread over the SMs: a stage ends at a
 // grid barrier, so its time is that of the CTA with the most items.
 //
-// Bound by the latency of the double operations at 16 warps per SM (128
-// registers; the item's constants lie in shared memory).  4 solves of 17-49
+// Bound by the CTA's barrier per heading (its warps wait there 6 times as long
+// as they take to issue) and the latency of the double operations, at 16 warps
+// per SM (128 registers; the item's constants lie in shared memory); the FP64
+// pipe is 30 % busy.  4 solves of 17-49
 // positions, 6.7e8 cell-stages: 56 ms on the cell-per-thread kernel, 22.7 ms
 // here; 32 solves, 7.7e9: 233 ms.  Handling two of the four cells at a time
 // keeps fewer values live but measured 22 % slower.

@@ -10,8 +10,9 @@
 // conversions per cell, with a range check on every quotient; here the
 // heading axis' are carried from step to step, the x axis' shared inside the
 // chunk, and the range checks are replaced by one test of the result
-// (relative5d_exact_walk.cuh): about 165 double operations per cell, which
-// bound it (64 per clock and SM): 1.82 ms per stage at 65x48x21x21 (4.0 ms
+// (relative5d_exact_walk.cuh): about 165 double operations per cell (64 per
+// clock and SM), whose dependent chains bound it with 10 to 16 warps per SM (FP64
+// pipe 38 to 42 % busy at 33x24x11x11): 1.82 ms per stage at 65x48x21x21 (4.0 ms
 // for the thread-per-cell kernel), of which the double operations are 0.85.
 #include "launch_shape.cuh"
 #include "relative5d_exact_walk.cuh"
@@ -202,7 +203,7 @@ cudaError_t launch(const RingArgs &args, size_t smem, int threads, cudaStream_t 
 // million cells, row padding not counted.  Near equal estimates the tiled one is
 // up to 17 % low, so it has to be 8 % below (B200, us per RK2 step in tiles and
 // per cell: 21x16x7x7 42.7, 38.1; 21x16x9x9 60.2, 59.0; 25x18x7x7 65.1, 53.2;
-// 25x18x9x9 64, 88; 33x24x11x11 207, 293; 65x48x21x21 3600, 8000.  It costs
+// 25x18x9x9 64, 88; 33x24x11x11 202, 293; 65x48x21x21 3630, 8000.  It costs
 // 23x16x7x7 44.7, 46.7).
 bool rel5_walk_exact_applies(const Rel5Grid &g, const Rel5Tile &t, const Rel5Stage &s) {
   if (g.xp % 4 != 0 || g.sy != g.xp ||
